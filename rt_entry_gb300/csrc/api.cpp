@@ -247,15 +247,34 @@ struct Plan {
 }  // namespace
 
 namespace rte {
-// The fewest warps per query that automatic teams use.  FP32 rows with pools
-// of up to 64 slots: their gathers bound the search, and two warps per query
-// keep twice the rows in flight, which is faster even when the batch fills
-// the GPU a few times over (measured on one GB300 with queries in leaf
-// order: 6-11 % at 10k queries, beams 16 to 64).  Above kTeamFloorLoad
-// times the resident warps one warp per query wins (9-20 % at 40k queries),
-// as it always does at beams 128 and 256 and for BF16 or FP8 rows.
-int team_floor(int prec, int L, int wpb) {
-  return prec == kPrecF32 && L <= 64 && wpb % 2 == 0 ? 2 : 1;
+// The fewest warps per query that automatic teams use, and up to how many
+// times the resident warps a batch keeps it (one warp per query above; the
+// larger teams of small batches come on top).  A team shares the gathers, so
+// two warps keep twice the rows in flight, and the last queries of a batch
+// take half the time; the leader's own work is not shared.  Measured on one
+// GB300, queries in leaf order, ms at K = 1 / 2 / 4 warps per query:
+//   rows of more than 4 chunks in registers (960 dims, 16 warps per SM, 2
+//     rows in flight a warp): FP32 beam 64, 1k queries 2.71 / 1.87 / 1.46, 4k
+//     6.78 / 4.74 / 3.80; FP8 beam 256 width 4, 4k 9.46 / 8.70 / 8.02: four;
+//   FP32 and FP8 rows, pools of up to 64 slots, 1M x 128: beam 32, 10k
+//     queries 1.21 / 1.00 / 1.10, 50k 3.67 / 3.61 / 4.38; beam 64, 50k 6.73 /
+//     6.71 / 8.25; FP8 beam 32, 10k 1.12 / 1.04 / 1.16: two, up to ten times;
+//   FP32 beam 128: 10k queries 2.75 / 2.62 / 3.40, 20k 4.52 / 4.65 / 6.20:
+//     two, up to three times;
+//   BF16 rows (tensor-core distances): beam 32, 7k queries 0.67 / 0.60 /
+//     0.68, 10k 0.82 / 0.80 / 0.92, 20k (beam 16) 0.91 / 0.92 / 1.11; beam
+//     128, 4k 0.98 / 1.04 / 1.40: two for pools of up to 64 slots, up to
+//     twice.
+// Wider pools are bound by the leader: one.  So are FP8 rows in the kernels
+// for any chunk count (d = 256 to 768, 6k queries: 1.48 / 1.61 / 1.74 to
+// 2.22 / 2.36 / 2.50).
+TeamFloor team_floor(int prec, int C, int kernel_chunks, int L, int wpb) {
+  if (kernel_chunks > 4 && wpb % 4 == 0) return {4, 1 << 20};
+  if (wpb % 2 != 0 || L > 128) return {1, 1};
+  if (prec == kPrecBF16 && C <= 4) return L <= 64 ? TeamFloor{2, 2} : TeamFloor{1, 1};
+  if (kernel_chunks == 0 && prec == kPrecFP8) return {1, 1};
+  if (L <= 64) return {2, 10};
+  return prec == kPrecF32 && kernel_chunks != 0 ? TeamFloor{2, 3} : TeamFloor{1, 1};
 }
 }  // namespace rte
 
@@ -326,8 +345,8 @@ rte_status plan_search(const rte_index* x, const rte_search_params* prm, int64_t
   const int64_t resident = (int64_t)x->num_sms * occ * pl.wpb;  // warps
   pl.team = team;
   if (team == 0) {  // automatic: spread a small batch's queries over the idle warps
-    pl.team = team_floor(pl.prec, pl.L, pl.wpb);
-    if (nq > kTeamFloorLoad * resident) pl.team = 1;
+    const TeamFloor f = team_floor(pl.prec, x->C, kc, pl.L, pl.wpb);
+    pl.team = nq > f.load * resident ? 1 : f.warps;
     while (pl.team < 8 && pl.wpb % (2 * pl.team) == 0 && nq * 2 * pl.team <= resident) pl.team *= 2;
   }
   const int64_t need = (nq * pl.team + pl.wpb - 1) / pl.wpb;

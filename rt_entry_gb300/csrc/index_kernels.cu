@@ -261,7 +261,7 @@ __global__ void interleave_rows(const float* __restrict__ src, int64_t n, int d,
       amax = fmaxf(amax, fabsf(v));
       const int64_t o = r * (32 * C) + interleaved_offset(c, lane, C);
       if (il32) il32[o] = v;
-      if (il16) il16[o] = __float2bfloat16_rn(v);
+      if (il16) il16[r * (32 * C) + bf16_offset(interleaved_offset(c, lane, C), C)] = __float2bfloat16_rn(v);
     }
     if (il8) {
       for (int off = 16; off >= 1; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
@@ -294,7 +294,7 @@ __global__ void lowp_from_il32(const float* __restrict__ il32, int64_t n, int C,
       const int64_t o = interleaved_offset(c, lane, C);
       const float v = s[o];
       amax = fmaxf(amax, fabsf(v));
-      if (il16) il16[r * (32 * C) + o] = __float2bfloat16_rn(v);
+      if (il16) il16[r * (32 * C) + bf16_offset((int)o, C)] = __float2bfloat16_rn(v);
     }
     if (il8) {
       for (int off = 16; off >= 1; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
@@ -335,7 +335,8 @@ __global__ void dequant_rows(const void* __restrict__ il, const float* __restric
       const int64_t o = r * (32 * C) + interleaved_offset(c, lane, C);
       float v;
       if (precision == 1) {
-        v = __uint_as_float((uint32_t)reinterpret_cast<const uint16_t*>(il)[o] << 16);
+        const int64_t o16 = r * (32 * C) + bf16_offset(interleaved_offset(c, lane, C), C);
+        v = __uint_as_float((uint32_t)reinterpret_cast<const uint16_t*>(il)[o16] << 16);
       } else {
         const uint8_t b = reinterpret_cast<const uint8_t*>(il)[o];
         v = fp8x2_to_float2((uint16_t)b).x * scale8[r];
@@ -566,7 +567,7 @@ __global__ void bf16_norms(const uint16_t* __restrict__ il16, int64_t n, int C,
     const uint16_t* row = il16 + r * 32 * C;
     double s = 0.0;
     for (int e = lane; e < 32 * C; e += 32) {
-      const double v = (double)__uint_as_float((uint32_t)row[e] << 16);
+      const double v = (double)__uint_as_float((uint32_t)row[bf16_offset(e, C)] << 16);
       s += v * v;
     }
     for (int off = 16; off >= 1; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);

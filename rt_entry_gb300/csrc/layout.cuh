@@ -11,8 +11,9 @@
 //   last odd chunk  -> 32 lanes x 1 value            (when C is odd)
 // Element offset of (chunk c, lane l) is interleaved_offset(c, l, C); a row
 // takes 32*C elements (dims >= d are stored as 0, which adds nothing to a
-// squared distance).  The same offsets are used for the FP32, BF16 and
-// FP8-E4M3 copies, so each copy is one coalesced gather per row.
+// squared distance).  The same offsets are used for the FP32 and FP8-E4M3
+// copies and, moved by bf16_offset, for the BF16 copy, so each copy is one
+// coalesced gather per row.
 #pragma once
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
@@ -26,6 +27,19 @@ __host__ __device__ inline int interleaved_offset(int c, int lane, int C) {
   if (c < 4 * n4) return 128 * (c >> 2) + 4 * lane + (c & 3);
   if (rem >= 2 && c < 4 * n4 + 2) return 128 * n4 + 2 * lane + (c - 4 * n4);
   return 128 * n4 + (rem >= 2 ? 64 : 0) + lane;
+}
+
+// Where the BF16 copy keeps interleaved element e of a row.  Rows of 2 to 4
+// chunks are read by the tensor-core distances: thread t (0..3) of a row
+// takes the 16-byte pieces 4i + t, i < C.  There the pieces of an even i and
+// of the next i lie side by side, so one 256-bit load gives the thread both
+// and four threads cover one whole 128-byte line: half the loads, and half
+// the L1 wavefronts, of 16-byte loads that each touch half of 8 lines.
+__host__ __device__ constexpr bool bf16_paired(int C) { return C >= 2 && C <= 4; }
+__host__ __device__ inline int bf16_offset(int e, int C) {
+  const int piece = e >> 3, i = piece >> 2, t = piece & 3;
+  if (!bf16_paired(C) || (i | 1) >= C) return e;
+  return ((i >> 1) * 8 + 2 * t + (i & 1)) * 8 + (e & 7);
 }
 
 template <int C>
@@ -56,6 +70,7 @@ __device__ __forceinline__ float bf16hi(uint32_t w) { return __uint_as_float(w &
 template <int C>
 __device__ __forceinline__ void load_interleaved_bf16(const __nv_bfloat16* __restrict__ row,
                                                       int lane, float (&v)[C]) {
+  static_assert(!bf16_paired(C), "rows of 2 to 4 chunks go to the tensor cores");
   constexpr int n4 = C / 4, rem = C % 4;
   const uint16_t* r = reinterpret_cast<const uint16_t*>(row);
 #pragma unroll

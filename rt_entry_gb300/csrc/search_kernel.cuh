@@ -29,6 +29,8 @@
 #include <cuda_fp8.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "layout.cuh"
 #include "search_types.h"
 
@@ -57,47 +59,73 @@ __device__ __forceinline__ uint32_t bloom_hash(int h, uint32_t x, uint32_t mask_
 
 struct Bloom {
   uint32_t* w;
+  uint32_t sw;          // w as a shared-space address
   uint32_t words_mask;  // words - 1
   uint32_t bits_mask;   // 32*words - 1
   int lw;               // log2(words)
   int nh;
   // set_bit / test_bit: word x % SIZE, bit x / SIZE (graph_search.cuh:7-28).
-  // The first kUnrolled hashes are unrolled, so their multipliers are
-  // constant-bank operands; further hashes (up to 10) run in a loop, which
-  // keeps the kernel's code small.
+  // The first kUnrolled hashes have no branch between them: a test computes
+  // all of them and issues its loads together, an id's hashes are computed
+  // once for its test and its add, and an id that is not to be added (or a
+  // hash beyond nh) ORs a zero instead of branching around the OR.  Measured
+  // on one GB300 with one warp on an SM, testing, adding and compacting 64
+  // ids: 1163 cycles with a branch per hash and around each add, 412 with
+  // predicated ORs, 254 this way.  Further hashes (up to 10) run in a loop.
   static constexpr int kUnrolled = 3;
-  __device__ __forceinline__ void add(uint32_t x) const {
+  __device__ __forceinline__ void set(uint32_t b, uint32_t on) const {
+    asm volatile("red.shared.or.b32 [%0], %1;" ::"r"(sw + 4 * (b & words_mask)), "r"(on << (b >> lw)) : "memory");
+  }
+  __device__ __forceinline__ uint32_t word(uint32_t b) const {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(sw + 4 * (b & words_mask)) : "memory");
+    return v;
+  }
+  __device__ __forceinline__ void hash(uint32_t x, uint32_t (&b)[kUnrolled]) const {
 #pragma unroll
-    for (int h = 0; h < kUnrolled; ++h) {
-      if (h >= nh) break;
-      uint32_t b = bloom_hash(h, x, bits_mask);
-      atomicOr(&w[b & words_mask], 1u << (b >> lw));
-    }
+    for (int h = 0; h < kUnrolled; ++h) b[h] = bloom_hash(h, x, bits_mask);
+  }
+  // Adds x where on = 1 (0: nothing is added); the warp's lanes all call it.
+  __device__ __forceinline__ void add(uint32_t (&b)[kUnrolled], uint32_t on) const {
+#pragma unroll
+    for (int h = 0; h < kUnrolled; ++h) set(b[h], h < nh ? on : 0u);
+  }
+  __device__ __forceinline__ void add(uint32_t x, uint32_t on) const {
+    uint32_t b[kUnrolled];
+    hash(x, b);
+    add(b, on);
 #pragma unroll 1
-    for (int h = kUnrolled; h < nh; ++h) {
-      uint32_t b = bloom_hash(h, x, bits_mask);
-      atomicOr(&w[b & words_mask], 1u << (b >> lw));
-    }
+    for (int h = kUnrolled; h < nh; ++h) set(bloom_hash(h, x, bits_mask), on);
+  }
+  __device__ __forceinline__ bool test(const uint32_t (&b)[kUnrolled]) const {
+    uint32_t v[kUnrolled];
+#pragma unroll
+    for (int h = 0; h < kUnrolled; ++h) v[h] = word(b[h]);
+    uint32_t ok = 1u;
+#pragma unroll
+    for (int h = 0; h < kUnrolled; ++h) ok &= (v[h] >> (b[h] >> lw)) | (h < nh ? 0u : 1u);
+    return ok != 0u;
   }
   __device__ __forceinline__ bool test(uint32_t x) const {
-    bool ok = true;
-#pragma unroll
-    for (int h = 0; h < kUnrolled; ++h) {
-      if (h >= nh) break;
-      uint32_t b = bloom_hash(h, x, bits_mask);
-      ok &= ((w[b & words_mask] >> (b >> lw)) & 1u) != 0;
-    }
+    uint32_t b[kUnrolled];
+    hash(x, b);
+    bool ok = test(b);
 #pragma unroll 1
     for (int h = kUnrolled; h < nh; ++h) {
-      uint32_t b = bloom_hash(h, x, bits_mask);
-      ok &= ((w[b & words_mask] >> (b >> lw)) & 1u) != 0;
+      const uint32_t c = bloom_hash(h, x, bits_mask);
+      ok &= ((word(c) >> (c >> lw)) & 1u) != 0u;
     }
     return ok;
   }
+  // The filter starts on a 16-byte boundary and holds at least 32 words.
   __device__ __forceinline__ void clear(int lane) const {
-    for (uint32_t i = lane; i <= words_mask; i += 32) w[i] = 0u;
+    uint4* w4 = reinterpret_cast<uint4*>(w);
+    for (uint32_t i = lane; i <= (words_mask >> 2); i += 32) w4[i] = make_uint4(0u, 0u, 0u, 0u);
   }
 };
+
+template <int V>
+using Const = std::integral_constant<int, V>;
 
 template <int N>
 __device__ __forceinline__ int pick(const int (&a)[N], int c) {
@@ -154,33 +182,31 @@ __host__ __device__ constexpr int qregs(int C) { return C == 0 ? 1 : C; }
 // 16 for the one-register beam-16 pool.  With DESC_FINAL the pair (a, a+sub)
 // is descending when a's 2*step block index is even, so the result is
 // descending, as the reference sorts its batch; otherwise the directions are
-// mirrored and the result is ascending.  Registers below KEEP_FROM are not
-// read after the sort (the merge reads only the last ones): the final step's
-// in-register stages skip them, which leaves every register that is read
-// unchanged.
-template <int NB, bool DESC_FINAL = true, int N = 32 * NB, int KEEP_FROM = 0>
+// mirrored and the result is ascending.  The stages are loops, not unrolled
+// code: the network runs only where equal distances or many candidates ask
+// for it (rank_candidates), and unrolled (36 stages x 8 registers for 256
+// slots) it made the kernels larger than the instruction cache, which on
+// one GB300 cost the 256-slot kernels 10 stalled cycles per issued
+// instruction.
+template <int NB, bool DESC_FINAL = true, int N = 32 * NB>
 __device__ __forceinline__ void sort_batch_desc(float (&d)[NB], int (&id)[NB], int lane) {
   constexpr int B = N;
-#pragma unroll
+#pragma unroll 1
   for (int step = 1; step <= B / 2; step <<= 1) {
 #pragma unroll
-    for (int sub = step; sub >= 1; sub >>= 1) {
-      if (sub >= 32) {
-        const int rs = sub >> 5;
+    for (int rs = NB / 2; rs >= 1; rs >>= 1) {
+      if (rs > (step >> 5)) continue;
 #pragma unroll
-        for (int j = 0; j < NB; ++j) {
-          if (j & rs) continue;
-          const bool desc = (((j << 5) & (2 * step)) == 0) == DESC_FINAL;
-          cx_regs(d[j], id[j], d[j + rs], id[j + rs], desc);
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < NB; ++j) {
-          if (step == B / 2 && j < KEEP_FROM) continue;  // dead after the sort
-          const bool desc = ((((j << 5) + lane) & (2 * step)) == 0) == DESC_FINAL;
-          cx_lanes(d[j], id[j], sub, desc, lane);
-        }
+      for (int j = 0; j < NB; ++j) {
+        if (j & rs) continue;
+        cx_regs(d[j], id[j], d[j + rs], id[j + rs], (((j << 5) & (2 * step)) == 0) == DESC_FINAL);
       }
+    }
+#pragma unroll 1
+    for (int sub = step < 16 ? step : 16; sub >= 1; sub >>= 1) {
+#pragma unroll
+      for (int j = 0; j < NB; ++j)
+        cx_lanes(d[j], id[j], sub, ((((j << 5) + lane) & (2 * step)) == 0) == DESC_FINAL, lane);
     }
   }
 }
@@ -191,15 +217,23 @@ template <int NL>
 __device__ __forceinline__ void half_clean(float (&pd)[pool_regs(NL)], int (&pi)[pool_regs(NL)], int lane) {
   constexpr int L = pool_slots(NL), PR = pool_regs(NL);
 #pragma unroll
-  for (int sub = L / 2; sub >= 1; sub >>= 1) {
-    if (sub >= 32) {
-      const int rs = sub >> 5;
+  for (int rs = PR / 2; rs >= 1; rs >>= 1) {
 #pragma unroll
-      for (int j = 0; j < PR; ++j) {
-        if (j & rs) continue;
-        cx_regs(pd[j], pi[j], pd[j + rs], pi[j + rs], false);
-      }
-    } else {
+    for (int j = 0; j < PR; ++j) {
+      if (j & rs) continue;
+      cx_regs(pd[j], pi[j], pd[j + rs], pi[j + rs], false);
+    }
+  }
+  constexpr int kFirst = L < 32 ? L / 2 : 16;
+  if constexpr (PR <= 2) {
+#pragma unroll
+    for (int sub = kFirst; sub >= 1; sub >>= 1) {
+#pragma unroll
+      for (int j = 0; j < PR; ++j) cx_lanes(pd[j], pi[j], sub, false, lane);
+    }
+  } else {
+#pragma unroll 1
+    for (int sub = kFirst; sub >= 1; sub >>= 1) {
 #pragma unroll
       for (int j = 0; j < PR; ++j) cx_lanes(pd[j], pi[j], sub, false, lane);
     }
@@ -208,11 +242,19 @@ __device__ __forceinline__ void half_clean(float (&pd)[pool_regs(NL)], int (&pi)
 
 // Pool/batch merge then the ascending half-cleaner (graph_search.cuh:921-957,
 // :1454-1493).  Pool slot L-n+i meets batch slot B-n+i (n = min(L,B)); both
-// are in the same lane.  The main loop skips a batch slot holding MAX.
+// are in the same lane.  The reference's main loop skips a batch slot holding
+// MAX; a pool slot is never above MAX, so the strict comparison does too.
 template <int NL, int NB>
 __device__ __forceinline__ void merge_pool(float (&pd)[pool_regs(NL)], int (&pi)[pool_regs(NL)],
                                            const float (&bd)[batch_regs(NB)],
-                                           const int (&bi)[batch_regs(NB)], bool skip_max, int lane) {
+                                           const int (&bi)[batch_regs(NB)], int lane) {
+  constexpr int PR = pool_regs(NL);
+  auto meet = [&](int pr, bool mine, float od, int oi) {
+    if (mine && pd[pr] > od) {
+      pd[pr] = od;
+      pi[pr] = oi;
+    }
+  };
   if constexpr (NB == 0) {
     // 16-slot batch: n = 16, batch slot i (lane i) meets pool slot L-16+i,
     // which is lane i of a 16-slot pool or lane 16+i of the last register
@@ -222,127 +264,364 @@ __device__ __forceinline__ void merge_pool(float (&pd)[pool_regs(NL)], int (&pi)
       od = __shfl_up_sync(kFull, od, 16);
       oi = __shfl_up_sync(kFull, oi, 16);
     }
-    constexpr int PR = pool_regs(NL);
-    const bool mine = NL == 0 ? lane < 16 : lane >= 16;
-    bool take = mine && pd[PR - 1] > od;
-    if (skip_max && od == kMaxDist) take = false;
-    if (take) {
-      pd[PR - 1] = od;
-      pi[PR - 1] = oi;
-    }
-    half_clean<NL>(pd, pi, lane);
+    meet(PR - 1, NL == 0 ? lane < 16 : lane >= 16, od, oi);
   } else if constexpr (NL == 0) {
     // 16-slot pool: pool slot i (lane i) meets batch slot B-16+i, which is
     // lane 16+i of the last batch register.
     const float od = __shfl_down_sync(kFull, bd[NB - 1], 16);
     const int oi = __shfl_down_sync(kFull, bi[NB - 1], 16);
-    bool take = lane < 16 && pd[0] > od;
-    if (skip_max && od == kMaxDist) take = false;
-    if (take) {
-      pd[0] = od;
-      pi[0] = oi;
-    }
-    half_clean<0>(pd, pi, lane);
+    meet(0, lane < 16, od, oi);
   } else {
     constexpr int NC = NL < NB ? NL : NB;
 #pragma unroll
-    for (int m = 0; m < NC; ++m) {
-      const int pr = NL - NC + m, br = NB - NC + m;
-      bool take = pd[pr] > bd[br];
-      if (skip_max && bd[br] == kMaxDist) take = false;
-      if (take) {
-        pd[pr] = bd[br];
-        pi[pr] = bi[br];
-      }
-    }
-    half_clean<NL>(pd, pi, lane);
+    for (int m = 0; m < NC; ++m) meet(NL - NC + m, true, bd[NB - NC + m], bi[NB - NC + m]);
   }
+  half_clean<NL>(pd, pi, lane);
 }
 
-// True when some batch distance lies strictly below the pool's largest
-// distance (slot L-1: lane 31 of the last register, or lane 15 of the
-// 16-slot pool).  When none does, the merge takes nothing -- it swaps only
-// where pool > batch, and every pool slot is <= the largest -- and the
-// half-cleaner then meets a pool that is still sorted ascending (the pool
-// leaves every merge sorted, and visiting a slot only negates its id), where
-// its strict comparisons swap nothing.  Sorting and merging such a batch
-// therefore leaves the pool unchanged, ids and order included, and
-// search_query skips both.
-template <int NL, int NB>
-__device__ __forceinline__ bool batch_can_enter(const float (&pd)[pool_regs(NL)],
-                                                const float (&bd)[batch_regs(NB)]) {
-  const float pmax = __shfl_sync(kFull, pd[pool_regs(NL) - 1], NL == 0 ? 15 : 31);
-  bool below = false;
-#pragma unroll
-  for (int j = 0; j < batch_regs(NB); ++j) below |= bd[j] < pmax;
-  return __any_sync(kFull, below);
-}
-
-// Candidates a batch may hold for merge_few.
-constexpr int kFewMax = 8;
-
-// Main-loop merge of a batch in which only a few slots (the candidates) hold
-// distances below the pool's largest, pmax.
-// The descending batch sort puts those candidates, if their distances are
-// pairwise distinct, in the batch's last slots in descending order whatever
+// ---- merging by rank ----
+// A batch's candidates are the distances strictly below the pool's largest.
+// When none is, the merge takes nothing -- it swaps only where pool > batch,
+// and every pool slot is <= the largest -- and the half-cleaner then meets a
+// pool that is still sorted ascending, where its strict comparisons swap
+// nothing: the pool stays as it is, ids and order included.
+//
+// With m candidates whose distances are pairwise distinct, the descending
+// batch sort puts them in the batch's last slots in descending order whatever
 // the network does with the other slots: the candidate of ascending rank r
 // lands in batch slot B-1-r, which the merge pairs with pool slot L-1-r.
 // Every other batch slot holds a distance >= the pool's largest, so its
-// comparison (pool > batch, strict) takes nothing.  Placing each candidate
-// against pool slot L-1-r by its rank and running the half-cleaner therefore
-// gives exactly the network's pool.  Returns false, changing nothing, when
-// two candidates tie (the network's order of equal distances then decides
-// which id lands where, so the caller runs it).
+// comparison takes nothing.  Placing each candidate against pool slot L-1-r
+// by its rank and running the half-cleaner (place_half_clean) therefore gives
+// exactly the network's pool.  If besides no candidate equals a pool slot and
+// no two pool slots (of real points) are equal, the half-cleaner's result is
+// the one ascending order of the L smallest, and the slots can be moved there
+// directly (place_direct).  Anything else -- ties, NaN, more candidates than
+// kept -- runs the reference's network, where the handling of equal keys
+// decides which id lands where.
+//
+// The candidates are compacted in shared memory and ranked one or two per
+// lane against broadcast reads: about 2 instructions per candidate, where
+// ranking them in the batch's slots by shuffles took 15 to 90, and no wide
+// network in the usual case.  On one GB300 this took the 256-slot pools
+// (10k queries, 500k x 96, BF16, beam 256, width 4) with the filter below from
+// 3.80 to 2.5 ms.
 template <int NL, int NB>
-__device__ __forceinline__ bool merge_few(float (&pd)[pool_regs(NL)], int (&pi)[pool_regs(NL)],
-                                          const float (&bd)[batch_regs(NB)], const int (&bi)[batch_regs(NB)],
-                                          float pmax, int lane) {
-  constexpr int BR = batch_regs(NB), PR = pool_regs(NL), L = pool_slots(NL);
-  unsigned cm[BR];
+__host__ __device__ constexpr int cands_per_lane() { return batch_regs(NB) >= 4 ? 2 : 1; }
+template <int NL, int NB>
+__host__ __device__ constexpr int cand_limit() {
+  constexpr int S = batch_slots(NB) > pool_slots(NL) ? batch_slots(NB) : pool_slots(NL);
+  return S < 32 ? S : 32 * cands_per_lane<NL, NB>();
+}
+
+// Candidates that are inserted one by one instead of ranked (pools of one or
+// two registers).
+constexpr int kInsertMax = 4;
+
+// One candidate into the sorted pool; eq is set if a slot equals it.
+template <int NL>
+__device__ __forceinline__ void insert_one(float (&pd)[pool_regs(NL)], int (&pi)[pool_regs(NL)], float v, int id,
+                                           bool& eq, int lane) {
+  constexpr int PR = pool_regs(NL);
+  float last_d = 0.0f;
+  int last_i = 0;
 #pragma unroll
-  for (int j = 0; j < BR; ++j) cm[j] = __ballot_sync(kFull, bd[j] < pmax);
-  // ascending rank of this lane's candidate in batch register t, 4 bits
-  // at bit 4t (ranks stay below kFewMax = 8; BR <= 8)
-  unsigned rank = 0;
-  bool tie = false;
+  for (int j = 0; j < PR; ++j) {
+    float up_d = __shfl_up_sync(kFull, pd[j], 1);
+    int up_i = __shfl_up_sync(kFull, pi[j], 1);
+    if (lane == 0) {
+      up_d = j > 0 ? last_d : v;
+      up_i = last_i;
+    }
+    if (j + 1 < PR) {
+      last_d = __shfl_sync(kFull, pd[j], 31);
+      last_i = __shfl_sync(kFull, pi[j], 31);
+    }
+    eq |= pd[j] == v;
+    if (pd[j] > v && (NL != 0 || lane < 16)) {
+      const bool moved = up_d > v;
+      pd[j] = moved ? up_d : v;
+      pi[j] = moved ? up_i : id;
+    }
+  }
+}
+
+// Merges the batch's candidates, (s_dist, s_ids)[0, n) below pmax, as far as
+// that can be done here: none or a few inserted ones leave the pool done and
+// give 0; otherwise they are compacted, ranked and left sorted ascending in
+// slots [0, m), padded with +inf to a multiple of four, and m is returned; or
+// -1, pool and arrays as they were, if the network has to run.
+template <int NL, int NB>
+__device__ __forceinline__ int rank_candidates(float (&pd)[pool_regs(NL)], int (&pi)[pool_regs(NL)], int* s_ids,
+                                               float* s_dist, int n, float pmax, bool ties, int lane) {
+  constexpr int PR = pool_regs(NL);
+  constexpr int KC = cands_per_lane<NL, NB>();
+  constexpr int kLim = cand_limit<NL, NB>();
+  const unsigned lt = (1u << lane) - 1u;
+  // the candidates of the first two blocks of 32, which hold most batches
+  constexpr int NK = batch_regs(NB) < 2 ? 1 : 2;
+  float d0[NK];
+  unsigned c0[NK];
+  int m = 0;
+  bool nan = false;
 #pragma unroll
-  for (int j = 0; j < BR; ++j) {
-    unsigned mask = cm[j];
-    while (mask) {
-      const int src = __ffs(mask) - 1;
-      mask &= mask - 1;
-      const float v = __shfl_sync(kFull, bd[j], src);
+  for (int t = 0; t < NK; ++t) {
+    const int i = 32 * t + lane;
+    d0[t] = i < n ? s_dist[i] : kMaxDist;
+    c0[t] = __ballot_sync(kFull, d0[t] < pmax);
+    nan |= d0[t] != d0[t];
+    m += __popc(c0[t]);
+  }
+#pragma unroll 1
+  for (int b = 32 * NK; b < n; b += 32) {
+    const float d = b + lane < n ? s_dist[b + lane] : kMaxDist;
+    nan |= d != d;
+    m += __popc(__ballot_sync(kFull, d < pmax));
+  }
+  if (m == 0) return 0;
+  if (__any_sync(kFull, nan)) return -1;
+  if constexpr (PR <= 2) {
+    // One to four candidates are inserted one after the other: every slot
+    // above the candidate moves up by one.  Without ties this is again the
+    // one ascending order of the L smallest; with one, the pool is put back.
+    if (m <= kInsertMax && !ties) {
+      float sd[PR];
+      int si[PR];
 #pragma unroll
-      for (int t = 0; t < BR; ++t) {
-        if ((cm[t] >> lane) & 1u) {
-          rank += bd[t] > v ? 1u << (4 * t) : 0u;
-          tie |= bd[t] == v && !(t == j && lane == src);
+      for (int j = 0; j < PR; ++j) {
+        sd[j] = pd[j];
+        si[j] = pi[j];
+      }
+      bool eq = false;
+#pragma unroll
+      for (int t = 0; t < NK; ++t) {
+        for (unsigned c = c0[t]; c; c &= c - 1) {
+          const int src = __ffs(c) - 1;
+          insert_one<NL>(pd, pi, __shfl_sync(kFull, d0[t], src), s_ids[32 * t + src], eq, lane);
         }
+      }
+#pragma unroll 1
+      for (int b = 32 * NK; b < n; b += 32) {
+        const float d = b + lane < n ? s_dist[b + lane] : kMaxDist;
+        for (unsigned c = __ballot_sync(kFull, d < pmax); c; c &= c - 1) {
+          const int src = __ffs(c) - 1;
+          insert_one<NL>(pd, pi, __shfl_sync(kFull, d, src), s_ids[b + src], eq, lane);
+        }
+      }
+      if (!__any_sync(kFull, eq)) return 0;
+#pragma unroll
+      for (int j = 0; j < PR; ++j) {
+        pd[j] = sd[j];
+        pi[j] = si[j];
+      }
+      return -1;
+    }
+  }
+  if (m > kLim) return -1;
+  // compact them, keeping the slots that this overwrites
+  float od[KC];
+  int oi[KC];
+#pragma unroll
+  for (int t = 0; t < KC; ++t) {
+    const int i = 32 * t + lane;
+    od[t] = i < n ? s_dist[i] : kMaxDist;
+    oi[t] = i < n ? s_ids[i] : 0;
+  }
+  int at = 0;
+#pragma unroll 1
+  for (int b = 0; b < n; b += 32) {
+    const int i = b + lane;
+    const float d = i < n ? s_dist[i] : kMaxDist;
+    const int id = i < n ? s_ids[i] : 0;
+    const unsigned mask = __ballot_sync(kFull, d < pmax);
+    __syncwarp();  // slots of this block and below have been read
+    if (d < pmax) {
+      s_dist[at + __popc(mask & lt)] = d;
+      s_ids[at + __popc(mask & lt)] = id;
+    }
+    at += __popc(mask);
+    __syncwarp();
+  }
+  bool ok;
+  {
+#pragma unroll
+    for (int t = 0; t < KC; ++t) {
+      const int i = 32 * t + lane;
+      if (i >= m && i < kLim) s_dist[i] = __int_as_float(0x7f800000);
+    }
+    __syncwarp();
+    float v[KC];
+    int id[KC], r[KC];
+#pragma unroll
+    for (int t = 0; t < KC; ++t) {
+      const int i = 32 * t + lane;
+      v[t] = i < kLim ? s_dist[i] : 0.0f;
+      id[t] = i < kLim ? s_ids[i] : 0;
+      r[t] = 0;
+    }
+#pragma unroll 2
+    for (int i = 0; i < m; i += 4) {
+      const float4 w = *reinterpret_cast<const float4*>(s_dist + i);
+#pragma unroll
+      for (int t = 0; t < KC; ++t)
+        r[t] += (w.x < v[t] ? 1 : 0) + (w.y < v[t] ? 1 : 0) + (w.z < v[t] ? 1 : 0) + (w.w < v[t] ? 1 : 0);
+    }
+    // distinct distances have distinct ranks
+    int ranks = 0;
+#pragma unroll
+    for (int t = 0; t < KC; ++t) {
+      unsigned bit[KC];
+#pragma unroll
+      for (int u = 0; u < KC; ++u) bit[u] = 32 * u + lane < m && (r[u] >> 5) == t ? 1u << (r[u] & 31) : 0u;
+      unsigned all = bit[0];
+      if constexpr (KC == 2) all |= bit[1];
+      ranks += __popc(__reduce_or_sync(kFull, all));
+    }
+    ok = ranks == m;
+    __syncwarp();
+    if (ok) {
+#pragma unroll
+      for (int t = 0; t < KC; ++t)
+        if (32 * t + lane < m) {
+          s_dist[r[t]] = v[t];
+          s_ids[r[t]] = id[t];
+        }
+    }
+  }
+  if (!ok) {
+    __syncwarp();
+#pragma unroll
+    for (int t = 0; t < KC; ++t) {
+      const int i = 32 * t + lane;
+      if (i < n) {
+        s_dist[i] = od[t];
+        s_ids[i] = oi[t];
       }
     }
   }
-  if (__any_sync(kFull, tie)) return false;
+  __syncwarp();
+  return ok ? m : -1;
+}
+
+// Ranked candidate r against pool slot L-1-r, then the half-cleaner.
+template <int NL, int NB>
+__device__ __forceinline__ void place_half_clean(float (&pd)[pool_regs(NL)], int (&pi)[pool_regs(NL)],
+                                                 const int* s_ids, const float* s_dist, int m, int lane) {
+  constexpr int PR = pool_regs(NL);
 #pragma unroll
-  for (int j = 0; j < BR; ++j) {
-    unsigned mask = cm[j];
-    while (mask) {
-      const int src = __ffs(mask) - 1;
-      mask &= mask - 1;
-      const float v = __shfl_sync(kFull, bd[j], src);
-      const int id = __shfl_sync(kFull, bi[j], src);
-      const int slot = L - 1 - (int)((__shfl_sync(kFull, rank, src) >> (4 * j)) & 15u);
-      if (lane == (slot & 31) && v != kMaxDist) {  // the main loop never takes a MAX slot
-#pragma unroll
-        for (int p = 0; p < PR; ++p) {
-          if (p == (slot >> 5) && pd[p] > v) {
-            pd[p] = v;
-            pi[p] = id;
-          }
-        }
+  for (int t = 0; t < cands_per_lane<NL, NB>(); ++t) {
+    const int r = 32 * t + (NL == 0 ? 15 : 31) - lane;
+    if (t < PR && r >= 0 && r < m) {
+      const float v = s_dist[r];
+      if (pd[PR - 1 - (t < PR ? t : 0)] > v) {
+        pd[PR - 1 - (t < PR ? t : 0)] = v;
+        pi[PR - 1 - (t < PR ? t : 0)] = s_ids[r];
       }
     }
   }
   half_clean<NL>(pd, pi, lane);
+}
+
+// Pools of 4 registers and more are merged directly: their half-cleaner is
+// 5 shuffle stages over every register, against two moves through shared
+// memory here.
+template <int NL>
+__host__ __device__ constexpr bool direct_pool() { return pool_regs(NL) >= 4; }
+
+// True when two neighbouring slots of the sorted pool hold equal distances
+// of real points.
+template <int NL>
+__device__ __forceinline__ bool pool_has_ties(const float (&pd)[pool_regs(NL)], int lane) {
+  constexpr int PR = pool_regs(NL);
+  bool tie = false;
+#pragma unroll
+  for (int j = 0; j < PR; ++j) {
+    float prev = __shfl_up_sync(kFull, pd[j], 1);
+    if (j > 0) {
+      const float last = __shfl_sync(kFull, pd[j > 0 ? j - 1 : 0], 31);
+      if (lane == 0) prev = last;
+    } else if (lane == 0) {
+      prev = kMaxDist;
+    }
+    tie |= prev == pd[j] && pd[j] != kMaxDist;
+  }
+  return __any_sync(kFull, tie);
+}
+
+// Moves the pool's slots and the m ranked candidates to their places in the
+// merged ascending order (the first L are kept).  Each candidate falls into
+// one pool register, found against the registers' last slots, and is compared
+// with that register alone; registers below the first candidate's stay as
+// they are.  Returns false, changing nothing, if a candidate equals a pool
+// slot.
+template <int NL, int NB>
+__device__ __forceinline__ bool place_direct(float (&pd)[pool_regs(NL)], int (&pi)[pool_regs(NL)], int* s_ids,
+                                             float* s_dist, int m, int lane) {
+  constexpr int L = pool_slots(NL), PR = pool_regs(NL), KC = cands_per_lane<NL, NB>();
+  float cv[KC];
+  int ci[KC], cp[KC], reg[KC];
+#pragma unroll
+  for (int t = 0; t < KC; ++t) {
+    const int r = 32 * t + lane;
+    cv[t] = r < m ? s_dist[r] : __int_as_float(0x7f800000);
+    ci[t] = r < m ? s_ids[r] : 0;
+    cp[t] = L;
+    reg[t] = r < m ? 0 : PR;
+  }
+#pragma unroll
+  for (int j = 0; j < PR - 1; ++j) {
+    const float last = __shfl_sync(kFull, pd[j], 31);
+#pragma unroll
+    for (int t = 0; t < KC; ++t) reg[t] += last < cv[t] ? 1 : 0;
+  }
+  int cnt[PR];        // candidates below each pool slot
+  int upto[PR];       // candidates in registers 0..j
+  bool eq = false;
+#pragma unroll
+  for (int j = 0; j < PR; ++j) {
+    int hi = 0;
+#pragma unroll
+    for (int t = 0; t < KC; ++t) hi += __popc(__ballot_sync(kFull, reg[t] <= j));
+    upto[j] = hi;
+    const int lo = j > 0 ? upto[j > 0 ? j - 1 : 0] : 0;
+    cnt[j] = lo;
+#pragma unroll 1
+    for (int r = lo; r < hi; ++r) {
+      const float c = s_dist[r];
+      const bool below = c < pd[j];
+      cnt[j] += below ? 1 : 0;
+      eq |= c == pd[j];
+      const int place = 32 * j + r + __popc(__ballot_sync(kFull, !below));
+#pragma unroll
+      for (int t = 0; t < KC; ++t)
+        if (32 * t + lane == r) cp[t] = place;
+    }
+  }
+  if (__any_sync(kFull, eq)) return false;
+  __syncwarp();  // every lane has read the candidates
+#pragma unroll
+  for (int t = 0; t < KC; ++t)
+    if (cp[t] < L) {
+      s_dist[cp[t]] = cv[t];
+      s_ids[cp[t]] = ci[t];
+    }
+#pragma unroll
+  for (int j = 0; j < PR; ++j) {
+    if (upto[j] == 0) continue;
+    const int p = 32 * j + lane + cnt[j];
+    if (p < L) {
+      s_dist[p] = pd[j];
+      s_ids[p] = pi[j];
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < PR; ++j) {
+    if (upto[j] == 0) continue;
+    pd[j] = s_dist[32 * j + lane];
+    pi[j] = s_ids[32 * j + lane];
+  }
+  __syncwarp();
   return true;
 }
 
@@ -416,12 +695,15 @@ __device__ __forceinline__ void team_sync(const Team& t) {
 
 // dist = |p|^2 + |q|^2 - 2 p.q, p the BF16 row, q the query rounded to BF16,
 // p.q from mma.sync m16n8k16 (BF16 inputs, exact products, FP32
-// accumulation).  A BF16 row (32*C values, 64*C bytes) is read as C pieces
-// of 64 bytes; thread t of each 4-thread group reads bytes [16t + 64i, +16)
-// of piece i -- storage elements 32i + 8t + j, j < 8 -- and uses them as the
-// MMA k-slots {2t, 2t+1, 2t+8, 2t+9} of k-tiles 2i (j < 4) and 2i+1 (j >= 4).
-// The query fragment comes from the query's own BF16 row at the same storage
-// positions, so each k pairs the base and query values of one dimension.
+// accumulation).  A BF16 row (32*C values, 64*C bytes) is C pieces of 64
+// interleaved bytes; thread t of each 4-thread group takes bytes
+// [16t + 64i, +16) of piece i -- interleaved elements 32i + 8t + j, j < 8 --
+// and uses them as the MMA k-slots {2t, 2t+1, 2t+8, 2t+9} of k-tiles 2i
+// (j < 4) and 2i+1 (j >= 4).  In memory the bytes of two pieces lie side by
+// side (bf16_offset), so one 256-bit load fetches both.
+// The query fragment comes from the query's own BF16 row at the same
+// interleaved positions, so each k pairs the base and query values of one
+// dimension.
 // With integer-valued data of magnitude < 2^8 every term is exact and the
 // distances equal the FP32 path's bit for bit.
 template <int C, int PREC, bool MMA = (PREC == kPrecBF16 && C >= 1 && C <= 4)>
@@ -467,7 +749,12 @@ __device__ __forceinline__ void make_query_extra(QueryExtra<C, kPrecBF16, true>&
   __syncwarp();
 }
 
-// L2 prefetch of the rows a warp is about to gather.  A batch of up to
+// L2 prefetch of the rows a warp is about to gather, where the rows are too
+// many to stay in L2 (SearchArgs::prefetch) and the warp has more than the
+// one group of rows that it loads at once anyway.  On one GB300, prefetching
+// always, or never: 10k queries over 96 MB of BF16 rows (beam 256, width 4)
+// 2.54 and 2.47 ms; 2,049 queries over 256 MB (beam 128) 0.582 and 0.600 ms;
+// one query as a team of 8 (one group a warp) 141 and 137 us.  A batch of up to
 // kPrefetchWhole bytes is prefetched at once.  A larger one goes through a
 // window of about kPrefetchBytes per warp: the first `ahead` rows of the
 // warp's share before its first group, then at each group the rows `ahead`
@@ -482,9 +769,17 @@ constexpr int kPrefetchWhole = 196608;
 __host__ __device__ constexpr int prefetch_ahead(int row_bytes, int G) {
   return kPrefetchBytes / row_bytes >= G ? kPrefetchBytes / row_bytes / G * G : G;
 }
+// Rows short enough that a batch of 256 is always prefetched whole: their
+// kernels have no window code.
+__host__ __device__ constexpr bool always_whole(int row_bytes) { return 256 * row_bytes <= kPrefetchWhole; }
 // Rows to prefetch before the first group: all n, or the window.
 __device__ __forceinline__ int prefetch_first(int n, int row_bytes, int ahead) {
   return n * row_bytes <= kPrefetchWhole ? n : ahead;
+}
+
+// Whether a member of a K-warp team prefetches at all.
+__device__ __forceinline__ bool prefetch_pays(const SearchArgs& a, int n, int G, int K) {
+  return a.prefetch && n > G * K;
 }
 
 // Prefetches rows [lr0, lr1) of member w's share of a K-warp team (groups
@@ -494,8 +789,10 @@ template <int G>
 __device__ __forceinline__ void prefetch_local(const char* rows, size_t row_bytes, int lines,
                                                const int* s_ids, int n, int lane, int w, int K, int lr0,
                                                int lr1) {
-  for (int i = lane + lr0 * lines; i < lr1 * lines; i += 32) {
-    const int lr = i / lines, line = i - lr * lines;
+  // each lane keeps one line of every (32 / lines)-th row
+  const int per = 32 / lines, r = lane / lines, line = lane - r * lines;
+  if (r >= per) return;
+  for (int lr = lr0 + r; lr < lr1; lr += per) {
     const int j = lr / G;
     const int row = G * (w + j * K) + (lr - j * G);
     if (row >= n) break;
@@ -505,8 +802,21 @@ __device__ __forceinline__ void prefetch_local(const char* rows, size_t row_byte
 
 // Distances of the n ids in s_ids[0..n) by the tensor cores, 8 rows per MMA
 // group: thread (g, t) supplies row g of the group as column g of the MMA's
-// B operand; the query is every row of A, so D[.][col] is the dot product of
-// row col, and lanes 0..3 hold the group's eight results.
+// B operand; the query is every row of A, so every lane of thread index t
+// holds the dot products of rows 2t and 2t+1: lane (0, t) finishes row 2t and
+// lane (1, t) row 2t+1, with one norm load and one store each.
+//
+// The LSU's wavefronts bound the 10k-query batches (85 % of its peak in ncu
+// on one GB300, 63 % issue).  A group of 8 rows of 128 dims took about 58:
+// 32 for four 16-byte loads over half of 8 lines each, 8 + 2 for the norms
+// and their ids, up to 16 for the query's fragments, 16 for its L2 prefetch.
+// 256-bit loads make the first 16.
+__device__ __forceinline__ void ldg256(const void* p, uint4& a, uint4& b) {
+  asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+      : "l"(p));
+}
+
 // One group of 8 rows from r0 (rows >= n are skipped).
 template <int C>
 __device__ __forceinline__ void mma_group(const SearchArgs& a, const QueryExtra<C, kPrecBF16, true>& qx,
@@ -514,51 +824,43 @@ __device__ __forceinline__ void mma_group(const SearchArgs& a, const QueryExtra<
   constexpr int kRowBytes = 64 * C;
   const char* rows = reinterpret_cast<const char*>(a.base_bf16);
   const int g = lane >> 2, t = lane & 3;
-  const int ra = r0 + g;
-  const int id = s_ids[ra < n ? ra : r0];
-  const char* p = rows + (size_t)id * kRowBytes + 16 * t;
+  uint4 qf[C];
+#pragma unroll
+  for (int i = 0; i < C; ++i) qf[i] = *reinterpret_cast<const uint4*>(qx.qs + 4 * t + 16 * i);
+  const int id = s_ids[r0 + g < n ? r0 + g : r0];
+  const char* p = rows + (size_t)id * kRowBytes;
   uint4 v[C];
+  if constexpr (bf16_paired(C)) {
 #pragma unroll
-  for (int i = 0; i < C; ++i) v[i] = __ldg(reinterpret_cast<const uint4*>(p + 64 * i));
-  // the norms of this lane's two output rows, loaded while the MMAs run
-  float pn[2] = {0.0f, 0.0f};
-  if (g == 0) {
+    for (int i = 0; i + 1 < C; i += 2) ldg256(p + 64 * i + 32 * t, v[i], v[i + 1]);
+    if constexpr (C & 1) v[C - 1] = __ldg(reinterpret_cast<const uint4*>(p + 64 * (C - 1) + 16 * t));
+  } else {
 #pragma unroll
-    for (int e = 0; e < 2; ++e)
-      if (r0 + 2 * t + e < n) pn[e] = __ldg(a.norm16 + s_ids[r0 + 2 * t + e]);
+    for (int i = 0; i < C; ++i) v[i] = __ldg(reinterpret_cast<const uint4*>(p + 64 * i + 16 * t));
   }
+  // the norm of the row this lane finishes, loaded while the MMAs run
+  const int row = r0 + 2 * t + g;
+  const bool mine = g < 2 && row < n;
+  const float pn = mine ? __ldg(a.norm16 + s_ids[row]) : 0.0f;
   float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
   for (int i = 0; i < C; ++i) {
-    const uint4 q = *reinterpret_cast<const uint4*>(qx.qs + 4 * t + 16 * i);
-    mma_bf16_16816(d, q.x, q.x, q.y, q.y, v[i].x, v[i].y);
-    mma_bf16_16816(d, q.z, q.z, q.w, q.w, v[i].z, v[i].w);
+    mma_bf16_16816(d, qf[i].x, qf[i].x, qf[i].y, qf[i].y, v[i].x, v[i].y);
+    mma_bf16_16816(d, qf[i].z, qf[i].z, qf[i].w, qf[i].w, v[i].z, v[i].w);
   }
-  if (g == 0) {
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int row = r0 + 2 * t + e;
-      if (row < n) s_dist[row] = __fmaf_rn(-2.0f, d[e], __fadd_rn(pn[e], qx.qn));
-    }
-  }
+  if (mine) s_dist[row] = __fmaf_rn(-2.0f, g == 0 ? d[0] : d[1], __fadd_rn(pn, qx.qn));
 }
 
 template <int C, bool TEAM>
 __device__ __forceinline__ void distances_mma(const SearchArgs& a, const QueryExtra<C, kPrecBF16, true>& qx,
                                               const int* s_ids, float* s_dist, int n, int lane, int w, int K) {
   constexpr int kRowBytes = 64 * C, kLines = (kRowBytes + 127) / 128;
-  constexpr int kAhead = prefetch_ahead(kRowBytes, 8);
+  static_assert(always_whole(kRowBytes), "no prefetch window");
   const char* rows = reinterpret_cast<const char*>(a.base_bf16);
   const int ws = TEAM ? w : 0, ks = TEAM ? K : 1;
-  const int first_rows = prefetch_first(n, kRowBytes, kAhead);
-  prefetch_local<8>(rows, kRowBytes, kLines, s_ids, n, lane, ws, ks, 0, first_rows);
-  const bool windowed = first_rows < n;
-  const int first = 8 * ws, step = 8 * ks;
-  int j = 0;
-  for (int r0 = first; r0 < n; r0 += step, ++j) {
-    if (windowed) prefetch_local<8>(rows, kRowBytes, kLines, s_ids, n, lane, ws, ks, kAhead + 8 * j, kAhead + 8 * j + 8);
-    mma_group<C>(a, qx, s_ids, s_dist, n, lane, r0);
-  }
+  if (prefetch_pays(a, n, 8, ks)) prefetch_local<8>(rows, kRowBytes, kLines, s_ids, n, lane, ws, ks, 0, n);
+#pragma unroll 1
+  for (int r0 = 8 * ws; r0 < n; r0 += 8 * ks) mma_group<C>(a, qx, s_ids, s_dist, n, lane, r0);
 }
 
 // ---- rows of a run-time chunk count (kernels built for any dimension) ----
@@ -571,7 +873,6 @@ struct SlabLoader;
 
 template <>
 struct SlabLoader<kPrecF32> {
-  static constexpr int kBytes = 4;
   const float* row;
   __device__ __forceinline__ void init(const SearchArgs& a, int id, size_t stride) { row = a.base + (size_t)id * stride; }
   __device__ __forceinline__ float4 quad(int off, int lane) const {
@@ -585,27 +886,28 @@ struct SlabLoader<kPrecF32> {
 
 template <>
 struct SlabLoader<kPrecBF16> {
-  static constexpr int kBytes = 2;
   const uint16_t* row;
+  int C;
   __device__ __forceinline__ void init(const SearchArgs& a, int id, size_t stride) {
     row = a.base_bf16 + (size_t)id * stride;
+    C = a.C;
   }
+  __device__ __forceinline__ const uint16_t* at(int e) const { return row + bf16_offset(e, C); }
   __device__ __forceinline__ float4 quad(int off, int lane) const {
-    const uint2 x = __ldg(reinterpret_cast<const uint2*>(row + off) + lane);
+    const uint2 x = __ldg(reinterpret_cast<const uint2*>(at(off + 4 * lane)));
     return make_float4(bf16lo(x.x), bf16hi(x.x), bf16lo(x.y), bf16hi(x.y));
   }
   __device__ __forceinline__ float2 pair(int off, int lane) const {
-    const uint32_t y = __ldg(reinterpret_cast<const unsigned int*>(row + off) + lane);
+    const uint32_t y = __ldg(reinterpret_cast<const unsigned int*>(at(off + 2 * lane)));
     return make_float2(bf16lo(y), bf16hi(y));
   }
   __device__ __forceinline__ float one(int off, int lane) const {
-    return __uint_as_float((uint32_t)__ldg(row + off + lane) << 16);
+    return __uint_as_float((uint32_t)__ldg(at(off + lane)) << 16);
   }
 };
 
 template <>
 struct SlabLoader<kPrecFP8> {
-  static constexpr int kBytes = 1;
   const uint8_t* row;
   float sc;
   __device__ __forceinline__ void init(const SearchArgs& a, int id, size_t stride) {
@@ -730,8 +1032,9 @@ __device__ __forceinline__ void distances_rt(const SearchArgs& a, const float* q
   const int ws = TEAM ? w : 0, ks = TEAM ? K : 1;
   const int ahead = prefetch_ahead((int)rb, G);
   const int first_rows = prefetch_first(n, (int)rb, ahead);
-  prefetch_local<G>(rows, rb, lines, s_ids, n, lane, ws, ks, 0, first_rows);
-  const bool windowed = first_rows < n;
+  const bool pays = prefetch_pays(a, n, G, ks);
+  if (pays) prefetch_local<G>(rows, rb, lines, s_ids, n, lane, ws, ks, 0, first_rows);
+  const bool windowed = pays && first_rows < n;
   const int first = G * ws, step = G * ks;
   int j = 0;
   for (int g0 = first; g0 < n; g0 += step, ++j) {
@@ -791,8 +1094,9 @@ __device__ __forceinline__ void prefetch_batch(const SearchArgs& a, const int* s
   constexpr int G = distance_group_size<C, PREC>();
   const int rb = 32 * (C == 0 ? a.C : C) * slab_bytes<PREC>();
   const int lines = (rb + 127) / 128;
-  prefetch_local<G>(search_rows<PREC>(a), rb, lines, s_ids, n, lane, 0, 1, 0,
-                    prefetch_first(n, rb, prefetch_ahead(rb, G)));
+  if (prefetch_pays(a, n, G, 1))
+    prefetch_local<G>(search_rows<PREC>(a), rb, lines, s_ids, n, lane, 0, 1, 0,
+                      prefetch_first(n, rb, prefetch_ahead(rb, G)));
 }
 
 // ---- helping in the tail ----
@@ -899,12 +1203,14 @@ __device__ __forceinline__ void distances(const SearchArgs& a, const float (&qv)
                                            : reinterpret_cast<const char*>(a.base_fp8);
     const int ws = TEAM ? w : 0, ks = TEAM ? K : 1;
     const int first_rows = prefetch_first(n, kRowBytes, kAhead);
-    prefetch_local<G>(rows, kRowBytes, kLines, s_ids, n, lane, ws, ks, 0, first_rows);
+    const bool pays = prefetch_pays(a, n, G, ks);
+    if (pays) prefetch_local<G>(rows, kRowBytes, kLines, s_ids, n, lane, ws, ks, 0, first_rows);
     const int first = G * ws, step = G * ks;
     auto group = [&](int g0) { regs_group<C, PREC>(a, qv, s_ids, s_dist, n, lane, g0); };
     // the window's loop is a copy of its own: the whole-batch loop keeps no
     // window state in the registers these rows fill
-    if (first_rows >= n) {
+    if (always_whole(kRowBytes) || !pays || first_rows >= n) {
+#pragma unroll 1
       for (int g0 = first; g0 < n; g0 += step) group(g0);
     } else {
       int j = 0;
@@ -916,29 +1222,25 @@ __device__ __forceinline__ void distances(const SearchArgs& a, const float (&qv)
   }
 }
 
-// Compact the valid batch ids (0 <= id < np) into s_ids in slot order,
-// compute their distances, and scatter them back (invalid slots -> MAX).
+// Appends the valid ids (0 <= id < np) of batch register j to the n ids in
+// s_ids, in slot order, and returns their new number; lane j keeps the
+// register's mask of valid slots in `slots`.
+__device__ __forceinline__ int compact_slot(int np, int id, int j, int n, int* s_ids, unsigned& slots, int lane) {
+  const bool v = id >= 0 && id < np;
+  const unsigned m = __ballot_sync(kFull, v);
+  if (v) s_ids[n + __popc(m & ((1u << lane) - 1u))] = id;
+  if (lane == j) slots = m;
+  return n + __popc(m);
+}
+
+// Distances of the n compacted ids in s_ids into s_dist.
 // With TEAM, the team's warps share the distances (team leader only).
 // Alone (not TEAM), with bs, idle warps of the block may help (tail).
 template <int C, int NB, int PREC, bool TEAM = false>
-__device__ __forceinline__ int batch_distances(const SearchArgs& a, const float (&qv)[qregs(C)],
-                                               const QueryExtra<C, PREC>& qx,
-                                               float (&bd)[batch_regs(NB)],
-                                               const int (&bi)[batch_regs(NB)], int* s_ids,
-                                               float* s_dist, int lane, const Team& t = Team(),
-                                               int q = 0, BlockShare* bs = nullptr) {
-  constexpr int BR = batch_regs(NB);
-  const unsigned lt = (1u << lane) - 1u;
-  int kidx[BR];
-  int n = 0;
-#pragma unroll
-  for (int j = 0; j < BR; ++j) {
-    const bool v = bi[j] >= 0 && bi[j] < a.np;
-    const unsigned m = __ballot_sync(kFull, v);
-    kidx[j] = v ? n + __popc(m & lt) : -1;
-    if (v) s_ids[kidx[j]] = bi[j];
-    n += __popc(m);
-  }
+__device__ __forceinline__ void batch_distances(const SearchArgs& a, const float (&qv)[qregs(C)],
+                                                const QueryExtra<C, PREC>& qx, const int* s_ids,
+                                                float* s_dist, int n, int lane, const Team& t = Team(),
+                                                int q = 0, BlockShare* bs = nullptr) {
   if constexpr (TEAM) {
     if (lane == 0) t.ctl[1] = n;
     team_sync(t);
@@ -956,12 +1258,52 @@ __device__ __forceinline__ int batch_distances(const SearchArgs& a, const float 
     }
     __syncwarp();
   }
-#pragma unroll
-  for (int j = 0; j < BR; ++j) bd[j] = kidx[j] >= 0 ? s_dist[kidx[j]] : kMaxDist;
-  __syncwarp();
-  return n;
 }
 
+// The reference's merge of a batch held compacted in (s_ids, s_dist): the
+// batch back in its slots (invalid ones hold MAX), sorted and merged by the
+// network.
+template <int NL, int NB>
+__device__ __forceinline__ void merge_network(float (&pd)[pool_regs(NL)], int (&pi)[pool_regs(NL)], int np,
+                                              const int* s_ids, const float* s_dist, unsigned slots,
+                                              int lane) {
+  constexpr int BR = batch_regs(NB);
+  const unsigned lt = (1u << lane) - 1u;
+  float bd[BR];
+  int bi[BR];
+  int at = 0;
+#pragma unroll
+  for (int j = 0; j < BR; ++j) {
+    const unsigned m = __shfl_sync(kFull, slots, j);
+    const bool v = (m >> lane) & 1u;
+    const int k = at + __popc(m & lt);
+    bd[j] = v ? s_dist[k] : kMaxDist;
+    bi[j] = v ? s_ids[k] : np;
+    at += __popc(m);
+  }
+  __syncwarp();
+  sort_batch_desc<BR, true, batch_slots(NB)>(bd, bi, lane);
+  merge_pool<NL, NB>(pd, pi, bd, bi, lane);
+}
+
+// The pool after a batch of n distances (compacted in s_ids / s_dist), m of
+// them ranked candidates (rank_candidates; -1: the network).  `ties` says
+// that two slots of the pool may be equal.
+template <int NL, int NB>
+__device__ __forceinline__ void merge_batch(float (&pd)[pool_regs(NL)], int (&pi)[pool_regs(NL)], int np,
+                                            int* s_ids, float* s_dist, int m, unsigned slots, bool& ties,
+                                            int lane) {
+  if (m == 0) return;
+  if constexpr (direct_pool<NL>()) {
+    if (m > 0 && !ties && place_direct<NL, NB>(pd, pi, s_ids, s_dist, m, lane)) return;
+  }
+  if (m > 0)
+    place_half_clean<NL, NB>(pd, pi, s_ids, s_dist, m, lane);
+  else
+    merge_network<NL, NB>(pd, pi, np, s_ids, s_dist, slots, lane);
+  __syncwarp();
+  ties = pool_has_ties<NL>(pd, lane);
+}
 
 // Exact FP32 rerank of the final pool for the reduced-precision paths: the
 // pool ids (visited marks dropped) get FP32 distances computed exactly as
@@ -975,15 +1317,15 @@ __device__ __forceinline__ void rerank_pool(const SearchArgs& a, const float (&q
                                             int lane, const Team& t = Team()) {
   constexpr int PR = pool_regs(NL);
   const unsigned lt = (1u << lane) - 1u;
-  int kidx[PR];
+  unsigned slots = 0;  // lane j: the valid slots of pool register j
   int n = 0;
 #pragma unroll
   for (int j = 0; j < PR; ++j) {
-    pi[j] = pi[j] < 0 ? -pi[j] : pi[j];
-    const bool v = pi[j] < a.np;
+    const int id = pi[j] < 0 ? -pi[j] : pi[j];
+    const bool v = id < a.np;
     const unsigned m = __ballot_sync(kFull, v);
-    kidx[j] = v ? n + __popc(m & lt) : -1;
-    if (v) s_ids[kidx[j]] = pi[j];
+    if (v) s_ids[n + __popc(m & lt)] = id;
+    if (lane == j) slots = m;
     n += __popc(m);
   }
   QueryExtra<C, kPrecF32> q32{};
@@ -998,8 +1340,16 @@ __device__ __forceinline__ void rerank_pool(const SearchArgs& a, const float (&q
     distances<C, kPrecF32>(a, qv, q32, s_ids, s_dist, n, lane);
     __syncwarp();
   }
+  int at = 0;
 #pragma unroll
-  for (int j = 0; j < PR; ++j) pd[j] = kidx[j] >= 0 ? s_dist[kidx[j]] : kMaxDist;
+  for (int j = 0; j < PR; ++j) {
+    const unsigned m = __shfl_sync(kFull, slots, j);
+    const bool v = (m >> lane) & 1u;
+    const int k = at + __popc(m & lt);
+    pd[j] = v ? s_dist[k] : kMaxDist;
+    pi[j] = v ? s_ids[k] : a.np;
+    at += __popc(m);
+  }
   __syncwarp();
   sort_batch_desc<PR, false, pool_slots(NL)>(pd, pi, lane);
 }
@@ -1012,6 +1362,15 @@ __device__ __forceinline__ void rerank_pool(const SearchArgs& a, const float (&q
 // The query's registers and shared-memory slot: FP32 chunks in registers
 // (C > 0; plus its BF16 row in q_slot for the tensor-core distances), or the
 // FP32 row in q_slot in the base's interleaved layout (C == 0).
+template <int C>
+__device__ __forceinline__ void load_query_chunks(const SearchArgs& a, int q, int lane, float (&qv)[qregs(C)]) {
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    const int dim = lane + 32 * c;
+    qv[c] = dim < a.d ? __ldg(a.queries + (size_t)q * a.qstride + dim) : 0.0f;
+  }
+}
+
 template <int C, int PREC>
 __device__ __forceinline__ void load_query(const SearchArgs& a, int q, int lane, float (&qv)[qregs(C)],
                                            QueryExtra<C, PREC>& qx, uint32_t* q_slot) {
@@ -1025,11 +1384,7 @@ __device__ __forceinline__ void load_query(const SearchArgs& a, int q, int lane,
     qx.qs = qs;
     __syncwarp();
   } else {
-#pragma unroll
-    for (int c = 0; c < C; ++c) {
-      const int dim = lane + 32 * c;
-      qv[c] = dim < a.d ? __ldg(a.queries + (size_t)q * a.qstride + dim) : 0.0f;
-    }
+    load_query_chunks<C>(a, q, lane, qv);
     if constexpr (PREC == kPrecBF16 && C <= 4) make_query_extra<C>(qx, qv, q_slot, lane);
   }
 }
@@ -1041,8 +1396,6 @@ __device__ __forceinline__ void search_query(const SearchArgs& a, int q, int lan
   constexpr int L = pool_slots(NL);
   constexpr int PR = pool_regs(NL);  // pool registers
   constexpr int BR = batch_regs(NB);  // batch registers
-  // the merge reads batch registers BR - min(PR, BR) .. BR-1 only
-  constexpr int kMergeFrom = BR - (PR < BR ? PR : BR);
   constexpr int B = batch_slots(NB);
   static_assert(R16 || NB > 0, "a 16-slot batch comes from a degree-16 graph");
   const int np = a.np;
@@ -1062,69 +1415,13 @@ __device__ __forceinline__ void search_query(const SearchArgs& a, int q, int lan
     pd[j] = kMaxDist;
     pi[j] = np;
   }
-  float bd[BR];
-  int bi[BR];
+  unsigned slots = 0;  // lane j: the valid slots of batch register j
+  bool ties = false;   // two pool slots may hold equal distances (merge_batch)
 
   bloom.clear(lane);
   __syncwarp();
 
-  // ---- entry phase (graph_search.cuh:479-959) ----
-  // kd-tree entries from several leaves (mode 1, max_hits H > 1, the
-  // reference's multi-hit entry, entry_helper.cu:5-241): every point of each
-  // leaf, leaf h in slots [h*cap, (h+1)*cap), -1 leaves as padding,
-  // max(L, H*cap) entry slots; the pool keeps the best L.
-  const int H = a.entry_mode == 1 ? a.max_hits : 1;
-  int hit = a.entry_mode != 0 ? __ldg(a.hits + (size_t)q * H) : 0;
-  if (hit < 0 || hit >= a.n_leaves) hit = 0;
-  const int32_t* lp = a.leaf_pids + (size_t)hit * a.leaf_cap;
-  // learned entries (mode 2): every point of the proposed leaf, then every
-  // point of the kd-tree leaf, max(L, both leaves) entry slots in all; the
-  // pool keeps the best L of them.  Modes 0 and 1 have L entry slots (:479).
-  int hit2 = a.entry_mode == 2 ? __ldg(a.hits2 + q) : -1;
-  if (hit2 >= a.n_leaves || hit2 == hit) hit2 = -1;
-  const int32_t* lp2 = a.leaf_pids + (size_t)(hit2 < 0 ? 0 : hit2) * a.leaf_cap;
-  const int n_first = a.leaf_cap;
-  const int n_second = hit2 >= 0 ? a.leaf_cap : 0;
-  const int n_entries = a.entry_mode == 2 ? max(L, n_first + n_second)
-                        : H > 1            ? max(L, H * a.leaf_cap)
-                                           : L;
-  uint32_t seed0 = (uint32_t)q * 64u + (uint32_t)lane;  // reference thread `lane`
-  uint32_t seed1 = seed0 + 32u;                           // reference thread `lane + 32`
-  const int n_ebatch = (n_entries + B - 1) / B;
-#pragma unroll 1
-  for (int it = 0; it < n_ebatch; ++it) {
-#pragma unroll
-    for (int j = 0; j < BR; ++j) {
-      const int slot = (j << 5) + lane;
-      const int pos = it * B + slot;
-      int id = np;
-      if (slot < B && pos < n_entries) {
-        if (a.entry_mode == 0) {
-          uint32_t& s = (j & 1) ? seed1 : seed0;
-          s = s * 1103515245u + 12345u;
-          id = (int)(s % (uint32_t)np);
-        } else if (H > 1) {
-          const int h = pos / a.leaf_cap, s = pos - h * a.leaf_cap;
-          const int lf = h < H ? __ldg(a.hits + (size_t)q * H + h) : -1;
-          if (lf >= 0 && lf < a.n_leaves) id = __ldg(a.leaf_pids + (size_t)lf * a.leaf_cap + s);
-        } else if (pos < n_first) {
-          id = __ldg(lp + pos);
-        } else if (hit2 >= 0 && pos < n_first + n_second) {
-          id = __ldg(lp2 + pos - n_first);
-        }
-        bloom.add((uint32_t)id);  // every entry, padding included (:490)
-      }
-      bi[j] = id;
-    }
-    __syncwarp();
-    c_entries += batch_distances<C, NB, PREC, TEAM>(a, qv, qx, bd, bi, s_ids, s_dist, lane, t, q, bs);
-    if (batch_can_enter<NL, NB>(pd, bd)) {
-      sort_batch_desc<BR, true, B, kMergeFrom>(bd, bi, lane);
-      merge_pool<NL, NB>(pd, pi, bd, bi, false, lane);
-    }
-  }
-
-  // ---- main loop (graph_search.cuh:961-1532) ----
+  // ---- main loop state (graph_search.cuh:961-1532) ----
   uint32_t tmp_flag = L >= 32 ? 0xFFFFFFFFu : ((1u << L) - 1u);  // (1 << min(L,32)) - 1 (:969)
   int iteration = 0;
   bool cz = false;  // this lane's check_zero (:967)
@@ -1145,142 +1442,264 @@ __device__ __forceinline__ void search_query(const SearchArgs& a, int q, int lan
     return __ballot_sync(kFull, pred);
   };
 
+  // The entry batches and the expansions share one loop, and so one copy of
+  // the distance and merge code: a trip gathers a batch's new ids into s_ids,
+  // from the entry list while entry batches are left, then from the lists of
+  // the nodes it selects.
+  // The number of entry batches comes from the parameters alone, so that the
+  // branch between the two is uniform to the compiler; a second leaf that
+  // equals the first only leaves a batch empty.
+  const int max_entries = a.entry_mode == 2                     ? max(L, 2 * a.leaf_cap)
+                          : a.entry_mode == 1 && a.max_hits > 1 ? max(L, a.max_hits * a.leaf_cap)
+                                                                : L;
+  const int n_ebatch = (max_entries + B - 1) / B;
 #pragma unroll 1
-  while (iter < a.max_iter) {
-    iter++;
-    // select up to W unvisited pool slots in pool order; mark them visited by
-    // negating the id (:986-1031).  nodes[s]: the s-th selected node (R >=
-    // 32); slot_node[j]: the node whose list fills this lane's slot of batch
-    // register j (R16).
-    int nodes[R16 ? 1 : BR];
-    int slot_node[R16 ? BR : 1];
-    int nsel = 0;
+  for (int eb = 0;;) {
+    int n = 0;
+    const bool entry = eb < n_ebatch;
+    if (entry) {
+      // ---- an entry batch (graph_search.cuh:479-959) ----
+      // The entry list's bounds are formed here for each batch, so that they
+      // hold no registers during the expansions.
+      // kd-tree entries from several leaves (mode 1, max_hits H > 1, the
+      // reference's multi-hit entry, entry_helper.cu:5-241): every point of
+      // each leaf, leaf h in slots [h*cap, (h+1)*cap), -1 leaves as padding,
+      // max(L, H*cap) entry slots; the pool keeps the best L.
+      const int H = a.entry_mode == 1 ? a.max_hits : 1;
+      int hit = a.entry_mode != 0 ? __ldg(a.hits + (size_t)q * H) : 0;
+      if (hit < 0 || hit >= a.n_leaves) hit = 0;
+      const int32_t* lp = a.leaf_pids + (size_t)hit * a.leaf_cap;
+      // learned entries (mode 2): every point of the proposed leaf, then
+      // every point of the kd-tree leaf, max(L, both leaves) entry slots in
+      // all; the pool keeps the best L of them.  Modes 0 and 1 have L entry
+      // slots (:479).
+      int hit2 = a.entry_mode == 2 ? __ldg(a.hits2 + q) : -1;
+      if (hit2 >= a.n_leaves || hit2 == hit) hit2 = -1;
+      const int32_t* lp2 = a.leaf_pids + (size_t)(hit2 < 0 ? 0 : hit2) * a.leaf_cap;
+      const int n_first = a.leaf_cap;
+      const int n_second = hit2 >= 0 ? a.leaf_cap : 0;
+      const int n_entries = a.entry_mode == 2 ? max(L, n_first + n_second)
+                            : H > 1            ? max(L, H * a.leaf_cap)
+                                               : L;
+      // mode 0: the LCGs of reference threads `lane` and `lane + 32`, moved
+      // past the earlier batches
+      uint32_t seed0 = (uint32_t)q * 64u + (uint32_t)lane;
+      uint32_t seed1 = seed0 + 32u;
+      auto lcg = [](uint32_t x) { return x * 1103515245u + 12345u; };
+      if (a.entry_mode == 0) {
 #pragma unroll 1
-    while (nsel < a.W && tmp_flag != 0) {
-      const int pos = __ffs(tmp_flag) - 1;
-      const int chunk = iteration;
-      const int v = __shfl_sync(kFull, pick<PR>(pi, chunk), pos);
-      if (lane == pos) {
+        for (int i = 0; i < eb * ((BR + 1) / 2); ++i) seed0 = lcg(seed0);
+#pragma unroll 1
+        for (int i = 0; i < eb * (BR / 2); ++i) seed1 = lcg(seed1);
+      }
+      const int base = eb * B;
+      slots = 0;
+#pragma unroll 2
+      for (int j = 0; j < BR; ++j) {
+        const int slot = (j << 5) + lane;
+        const int pos = base + slot;
+        int id = np;
+        if (slot < B && pos < n_entries) {
+          if (a.entry_mode == 0) {
+            const uint32_t s = lcg((j & 1) ? seed1 : seed0);
+            if (j & 1)
+              seed1 = s;
+            else
+              seed0 = s;
+            id = (int)(s % (uint32_t)np);
+          } else if (H > 1) {
+            const int h = pos / a.leaf_cap, s = pos - h * a.leaf_cap;
+            const int lf = h < H ? __ldg(a.hits + (size_t)q * H + h) : -1;
+            if (lf >= 0 && lf < a.n_leaves) id = __ldg(a.leaf_pids + (size_t)lf * a.leaf_cap + s);
+          } else if (pos < n_first) {
+            id = __ldg(lp + pos);
+          } else if (hit2 >= 0 && pos < n_first + n_second) {
+            id = __ldg(lp2 + pos - n_first);
+          }
+        }
+        bloom.add((uint32_t)id, slot < B && pos < n_entries ? 1u : 0u);  // every entry, padding included (:490)
+        n = compact_slot(np, id, j, n, s_ids, slots, lane);
+      }
+      c_entries += n;
+      ++eb;
+    } else {
+      if (iter >= a.max_iter) break;
+      iter++;
+      // select up to W unvisited pool slots in pool order; mark them visited
+      // by negating the id (:986-1031).  The slots chosen in one register are
+      // taken together; the s-th selected node is kept by lane s.
+      int my_node = np;
+      int nsel = 0;
+      const unsigned lt = (1u << lane) - 1u;
+#pragma unroll 1
+      while (nsel < a.W && tmp_flag != 0) {
+        const int v = pick<PR>(pi, iteration);
+        const int rank = __popc(tmp_flag & lt);
+        const bool chosen = ((tmp_flag >> lane) & 1u) && rank < a.W - nsel;
+        const unsigned took = __ballot_sync(kFull, chosen);
+        const int nt = __popc(took);
+        if (a.W == 1) {
+          my_node = __shfl_sync(kFull, v, __ffs(took) - 1);
+          my_node = my_node < 0 ? -my_node : my_node;
+        } else {
+          if (chosen) s_ids[nsel + rank] = v < 0 ? -v : v;
+          __syncwarp();
+          if (lane >= nsel && lane < nsel + nt) my_node = s_ids[lane];
+          __syncwarp();
+        }
 #pragma unroll
         for (int j = 0; j < PR; ++j)
-          if (j == chunk) pi[j] = -pi[j];
+          if (j == iteration && chosen) pi[j] = -pi[j];
+        tmp_flag &= ~took;
+        nsel += nt;
+        if (nsel == a.W) break;
+        while (tmp_flag == 0 && iteration < PR) {
+          iteration++;
+          tmp_flag = scan(iteration);
+        }
       }
-      tmp_flag &= ~(1u << pos);
-      const int node = v < 0 ? -v : v;
-      if constexpr (R16) {
-#pragma unroll
-        for (int j = 0; j < BR; ++j)
-          if ((((j << 5) + lane) >> 4) == nsel) slot_node[j] = node;
-        if (lane == 0) c_expanded += node < np ? 1 : 0;
-      } else {
-#pragma unroll
-        for (int s = 0; s < BR; ++s)
-          if (s == nsel) nodes[s] = node;
+      if (nsel == 0) break;
+      c_expanded += __popc(__ballot_sync(kFull, lane < nsel && my_node < np));
+      // the next unvisited pool node, often the next iteration's choice: its
+      // adjacency row into L2 while this iteration's rows are gathered (the
+      // reduced-precision paths, which latency bounds; the FP32 path is
+      // bandwidth-bound and loses more to the prefetches that miss)
+      if (PREC != kPrecF32 && tmp_flag != 0) {
+        const int u = __shfl_sync(kFull, pick<PR>(pi, iteration), __ffs(tmp_flag) - 1);
+        if (u >= 0 && u < np && lane < ((R + 31) >> 5))
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(a.graph + (size_t)u * R + 32 * lane));
       }
-      nsel++;
-      if (nsel == a.W) break;
-      while (tmp_flag == 0 && iteration < PR) {
-        iteration++;
-        tmp_flag = scan(iteration);
-      }
-    }
-    if (nsel == 0) break;
-    // the next unvisited pool node, often the next iteration's choice: its
-    // adjacency row into L2 while this iteration's rows are gathered (the
-    // reduced-precision paths, which latency bounds; the FP32 path is
-    // bandwidth-bound and loses more to the prefetches that miss)
-    if (PREC != kPrecF32 && tmp_flag != 0) {
-      const int u = __shfl_sync(kFull, pick<PR>(pi, iteration), __ffs(tmp_flag) - 1);
-      if (u >= 0 && u < np && lane < ((R + 31) >> 5))
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(a.graph + (size_t)u * R + 32 * lane));
-    }
 
-    // neighbour rows of the selected nodes (:995-1010); a node id >= np
-    // expands nothing (the reference would read past the graph)
-#pragma unroll
-    for (int j = 0; j < BR; ++j) {
-      int id = np;
+      // neighbour rows of the selected nodes (:995-1010); a node id >= np
+      // expands nothing (the reference would read past the graph)
       if constexpr (R16) {
-        const int slot = (j << 5) + lane;
-        if (slot < B && (slot >> 4) < nsel) {
-          const int node = slot_node[j];
-          if (node < np) id = __ldg(a.graph + (size_t)node * 16 + (slot & 15));
+        // a register holds the lists of two nodes, one per half
+        int* s_raw = reinterpret_cast<int*>(s_dist);  // free until the distances
+#pragma unroll
+        for (int j = 0; j < BR; ++j) {
+          const int slot = (j << 5) + lane;
+          const int node = __shfl_sync(kFull, my_node, slot >> 4);
+          const int id = slot < B && node < np ? __ldg(a.graph + (size_t)node * 16 + (slot & 15)) : np;
+          if (slot < B) s_raw[slot] = id;
         }
-      } else {
-        const int s = j >> nr_shift;
-        if (s < nsel) {
-          const int node = pick<BR>(nodes, s);
-          if (node < np) id = __ldg(a.graph + (size_t)node * R + ((j - s * NR) << 5) + lane);
-        }
-      }
-      bi[j] = id;
-    }
-    // canonical rule: every test of one list sees the filter before any add
-    // of that list; lists in selection order
-    if constexpr (R16) {
+        // canonical rule: every test of one list sees the filter before any
+        // add of that list; lists in selection order
+        slots = 0;
 #pragma unroll 1
-      for (int s = 0; s < nsel; ++s) {
-        bool pass[BR];
-#pragma unroll
-        for (int j = 0; j < BR; ++j) {
-          pass[j] = false;
-          if ((((j << 5) + lane) >> 4) == s) pass[j] = bi[j] != np && !bloom.test((uint32_t)bi[j]);
+        for (int j = 0; 2 * j < nsel; ++j) {
+          const int slot = (j << 5) + lane;
+          const int id = slot < B ? s_raw[slot] : np;
+          bool pass = false;
+#pragma unroll 1
+          for (int half = 0; half < 2; ++half) {
+            const bool seen = bloom.test((uint32_t)id);
+            const bool p = ((lane >> 4) == half) & (id != np) & !seen;
+            __syncwarp();
+            bloom.add((uint32_t)id, p ? 1u : 0u);
+            pass |= p;
+            __syncwarp();
+          }
+          n = compact_slot(np, pass ? id : np, j, n, s_ids, slots, lane);
         }
-        __syncwarp();
+      } else {
+        // canonical rule: every test of one list (NR registers) sees the
+        // filter before any add of that list; lists in selection order.
+        // Up to KB registers are filtered together, list by list, with their
+        // hashes computed ahead.
+        constexpr int KB = BR < 4 ? BR : 4;
+        slots = 0;
+        auto filter = [&](const int (&bi)[KB], int j0) {
+          uint32_t hb[KB][Bloom::kUnrolled];
+#pragma unroll
+          for (int j = 0; j < KB; ++j) bloom.hash((uint32_t)bi[j], hb[j]);
+          auto list = [&](auto first, auto count) {
+            constexpr int F = decltype(first)::value, N = decltype(count)::value;
+            bool pass[N];
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+              const bool seen = bloom.test(hb[F + j]);
+              pass[j] = (bi[F + j] != np) & !seen;
+            }
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+              bloom.add(hb[F + j], pass[j] ? 1u : 0u);
+              n = compact_slot(np, pass[j] ? bi[F + j] : np, j0 + F + j, n, s_ids, slots, lane);
+            }
+            __syncwarp();
+          };
+          if (NR >= KB) {
+            list(Const<0>(), Const<KB>());
+          } else if (KB == 4 && NR == 2) {
+            list(Const<0>(), Const<KB == 4 ? 2 : 1>());
+            list(Const<KB == 4 ? 2 : 0>(), Const<KB == 4 ? 2 : 1>());
+          } else {
+            list(Const<0>(), Const<1>());
+            if constexpr (KB > 1) list(Const<1>(), Const<1>());
+            if constexpr (KB > 2) {
+              list(Const<2>(), Const<1>());
+              list(Const<3>(), Const<1>());
+            }
+          }
+        };
+        int bi[BR];
 #pragma unroll
         for (int j = 0; j < BR; ++j) {
-          if ((((j << 5) + lane) >> 4) == s) {
-            if (pass[j])
-              bloom.add((uint32_t)bi[j]);
-            else
-              bi[j] = np;
+          const int s = j >> nr_shift;
+          const int node = __shfl_sync(kFull, my_node, s);
+          bi[j] = node < np ? __ldg(a.graph + (size_t)node * R + ((j - s * NR) << 5) + lane) : np;
+        }
+        if (BR <= 4 && bloom.nh <= Bloom::kUnrolled) {
+          if constexpr (BR <= 4) filter(bi, 0);
+        } else {
+          // more registers or hashes: the ids wait in s_dist (free until the
+          // distances), where a loop reads them; unrolled over all registers
+          // and lists, the filter's code alone outgrew the instruction cache
+          int* s_raw = reinterpret_cast<int*>(s_dist);
+#pragma unroll
+          for (int j = 0; j < BR; ++j) s_raw[(j << 5) + lane] = bi[j];
+          if (NR <= KB && bloom.nh <= Bloom::kUnrolled) {
+#pragma unroll 1
+            for (int j0 = 0; j0 < nsel * NR; j0 += KB) {
+              int part[KB];
+#pragma unroll
+              for (int j = 0; j < KB; ++j) part[j] = s_raw[((j0 + j) << 5) + lane];
+              filter(part, j0);
+            }
+          } else {
+#pragma unroll 1
+            for (int s = 0; s < nsel; ++s) {
+              unsigned pass = 0;
+#pragma unroll 1
+              for (int r = 0; r < NR; ++r) {
+                const int id = s_raw[((s * NR + r) << 5) + lane];
+                const bool seen = bloom.test((uint32_t)id);
+                if (id != np && !seen) pass |= 1u << r;
+              }
+              __syncwarp();
+#pragma unroll 1
+              for (int r = 0; r < NR; ++r) {
+                const int j = s * NR + r;
+                const int id = s_raw[(j << 5) + lane];
+                const uint32_t p = (pass >> r) & 1u;
+                bloom.add((uint32_t)id, p);
+                n = compact_slot(np, p ? id : np, j, n, s_ids, slots, lane);
+              }
+              __syncwarp();
+            }
           }
         }
-        __syncwarp();
       }
-    } else {
-#pragma unroll
-      for (int s = 0; s < BR; ++s) {
-        if (s >= nsel) break;
-        if (lane == 0) c_expanded += pick<BR>(nodes, s) < np ? 1 : 0;
-        bool pass[BR];
-#pragma unroll
-        for (int j = 0; j < BR; ++j) {
-          pass[j] = false;
-          if ((j >> nr_shift) == s) pass[j] = bi[j] != np && !bloom.test((uint32_t)bi[j]);
-        }
-        __syncwarp();
-#pragma unroll
-        for (int j = 0; j < BR; ++j) {
-          if ((j >> nr_shift) == s) {
-            if (pass[j])
-              bloom.add((uint32_t)bi[j]);
-            else
-              bi[j] = np;
-          }
-        }
-        __syncwarp();
-      }
+      c_dists += n;
     }
 
-    c_dists += batch_distances<C, NB, PREC, TEAM>(a, qv, qx, bd, bi, s_ids, s_dist, lane, t, q, bs);
-    {
-      // batch slots below the pool's largest distance: none -> the merge
-      // changes nothing (batch_can_enter); a few distinct ones -> placed
-      // by rank (merge_few); otherwise the reference's network
-      const float pmax = __shfl_sync(kFull, pd[PR - 1], NL == 0 ? 15 : 31);
-      int m = 0;
-      bool nan = false;
-#pragma unroll
-      for (int j = 0; j < BR; ++j) {
-        m += __popc(__ballot_sync(kFull, bd[j] < pmax));
-        nan |= bd[j] != bd[j];
-      }
-      if (m > 0 && (m > kFewMax || __any_sync(kFull, nan) || !merge_few<NL, NB>(pd, pi, bd, bi, pmax, lane))) {
-        sort_batch_desc<BR, true, B, kMergeFrom>(bd, bi, lane);
-        merge_pool<NL, NB>(pd, pi, bd, bi, true, lane);
-      }
-    }
+    batch_distances<C, NB, PREC, TEAM>(a, qv, qx, s_ids, s_dist, n, lane, t, q, bs);
+    // the pool's largest distance: lane 31 of the last register, or lane 15
+    // of the 16-slot pool
+    const float pmax = __shfl_sync(kFull, pd[PR - 1], NL == 0 ? 15 : 31);
+    const int m = rank_candidates<NL, NB>(pd, pi, s_ids, s_dist, n, pmax, ties, lane);
+    merge_batch<NL, NB>(pd, pi, np, s_ids, s_dist, m, slots, ties, lane);
+    if (entry) continue;
 
     bool any = false;
 #pragma unroll 1
@@ -1295,10 +1714,11 @@ __device__ __forceinline__ void search_query(const SearchArgs& a, int q, int lan
       __syncwarp();
       bloom.clear(lane);
       __syncwarp();
-#pragma unroll
+#pragma unroll 1
       for (int j = 0; j < PR; ++j) {
-        const int id = pi[j] < 0 ? -pi[j] : pi[j];
-        if (id < np) bloom.add((uint32_t)id);
+        const int v = pick<PR>(pi, j);
+        const int id = v < 0 ? -v : v;
+        bloom.add((uint32_t)id, id < np ? 1u : 0u);
       }
       __syncwarp();
       hash_iteration = 0;
@@ -1308,8 +1728,12 @@ __device__ __forceinline__ void search_query(const SearchArgs& a, int q, int lan
   }
 
   // ---- exact FP32 rerank of the final pool (precision paths) ----
-  if (PREC != kPrecF32 && a.rerank)
+  if (PREC != kPrecF32 && a.rerank) {
+    // the tensor-core distances read the query from shared memory: its FP32
+    // chunks hold no registers until here
+    if constexpr (PREC == kPrecBF16 && C >= 1 && C <= 4) load_query_chunks<C>(a, q, lane, qv);
     rerank_pool<C, NL, TEAM>(a, qv, reinterpret_cast<const float*>(q_slot), pd, pi, s_ids, s_dist, lane, t);
+  }
   if constexpr (TEAM) {  // releases the helpers
     if (lane == 0) t.ctl[1] = -1;
     team_sync(t);
@@ -1406,11 +1830,7 @@ __device__ __noinline__ void help_block(const SearchArgs a, uint32_t* smem, int 
       if constexpr (C == 0) {
         qx.qs = reinterpret_cast<const float*>(lslot);
       } else {
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-          const int dim = lane + 32 * c;
-          qv[c] = dim < a.d ? __ldg(a.queries + (size_t)q * a.qstride + dim) : 0.0f;
-        }
+        load_query_chunks<C>(a, q, lane, qv);
         if constexpr (PREC == kPrecBF16 && C <= 4) {
           qx.qs = lslot;
           qx.qn = *reinterpret_cast<volatile float*>(&d.qn);
@@ -1463,6 +1883,7 @@ __global__ void __launch_bounds__(256, search_min_blocks(C, NL, NB)) search_kern
   uint32_t* wbase = smem + (size_t)wib * per_warp;
   Bloom bloom;
   bloom.w = wbase;
+  bloom.sw = (uint32_t)__cvta_generic_to_shared(wbase);
   bloom.words_mask = (uint32_t)a.bloom_words - 1u;
   bloom.bits_mask = ((uint32_t)a.bloom_words << 5) - 1u;
   bloom.lw = __ffs(a.bloom_words) - 1;
@@ -1489,7 +1910,7 @@ __global__ void __launch_bounds__(256, search_min_blocks(C, NL, NB)) search_kern
 }
 
 // search_kernel with teams of K warps per query (Team): K = a.team, or,
-// for a.team < 0, at least -a.team (one above kTeamFloorLoad times the
+// for a.team < 0, at least -a.team (one above a.team_load times the
 // grid's warps) and otherwise the most (up to 8) that the live query count
 // leaves room for in the grid.  K = 1 runs as a team of one.  A kernel of its own, so
 // that the single-warp kernel's code and register allocation stay as they
@@ -1510,6 +1931,7 @@ __global__ void __launch_bounds__(256, search_min_blocks(C, NL, NB)) search_kern
   uint32_t* wbase = smem + (size_t)wib * per_warp;
   Bloom bloom;
   bloom.w = wbase;
+  bloom.sw = (uint32_t)__cvta_generic_to_shared(wbase);
   bloom.words_mask = (uint32_t)a.bloom_words - 1u;
   bloom.bits_mask = ((uint32_t)a.bloom_words << 5) - 1u;
   bloom.lw = __ffs(a.bloom_words) - 1;
@@ -1520,7 +1942,7 @@ __global__ void __launch_bounds__(256, search_min_blocks(C, NL, NB)) search_kern
   if (K < 0) {  // at least -a.team warps, then as many as the live batch leaves room for
     const long long total = (long long)gridDim.x * wpb;
     K = -a.team;
-    if ((long long)nq > kTeamFloorLoad * total) K = 1;  // the floor holds for moderate batches only
+    if ((long long)nq > a.team_load * total) K = 1;  // the floor holds for moderate batches only
     while (K < 8 && wpb % (2 * K) == 0 && (long long)nq * 2 * K <= total) K *= 2;
   }
   if (K < 1 || K > 8 || wpb % K != 0) K = 1;

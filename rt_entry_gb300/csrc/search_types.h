@@ -29,10 +29,6 @@ RTE_HD constexpr int query_slot_words_for(int C, int chunks) {
 // (a power of two >= 32 words), the compaction words (2 x 16..256) and the
 // query slot (64 or 32 x chunks words) are all multiples of 4 words.
 constexpr int kTeamCtlWords = 4;
-// Automatic teams keep their floor of warps per query (more than one: FP32
-// rows with pools of up to 64 slots) only while a batch is at most this
-// many times the resident warps; above it one warp per query is faster.
-constexpr int kTeamFloorLoad = 3;
 // Shared memory a search block keeps after its warps' regions: the tail
 // helping state (a count of idle warps and one phase descriptor per warp,
 // search_kernel.cuh's BlockShare).  Every launch reserves it.
@@ -65,9 +61,12 @@ struct SearchArgs {
   int C;                    // chunks of 32 dims per row (set by launch_search)
   int team;                 // warps per query: 0 or 1 alone, 2/4/8 a team, < 0 chosen
                             // by the kernel from the live query count, at least -team
+                            // up to team_load times the grid's warps
+  int team_load;
   int* err;                 // device word set to a non-zero code when a bounded wait runs out, or null
   const int32_t* order;     // [nq] the order in which queries are taken (a permutation), or null
   int order_min;            // the order is read only for more than this many queries
+  int prefetch;             // rows are prefetched into L2 (set by launch_search: too many to stay there)
 };
 
 }  // namespace rte
