@@ -252,9 +252,9 @@ void subtree_classes(const KdTree& t, int depth, std::vector<int32_t>& leaf_clas
 // Buffers of one optimisation step on a batch of M rows.
 struct StepBufs {
   DevBuf<uint16_t> H1, H2, dZ, dZT, H2T, W3T, dH2, dH2T, H1T, W2T, dH1, dH1T, XT;
-  DevBuf<float> Z, dH2f, dH1f, loss, colpart;
+  DevBuf<float> Z, dH2f, dH1f, loss, colpart[3];
   rte_status alloc(int M, int H, int C, int dp) {
-    RTE_CUDA(colpart.alloc((size_t)col_sum_slices(M) * std::max(H, C)));
+    for (int l = 0; l < 3; ++l) RTE_CUDA(colpart[l].alloc((size_t)col_sum_slices(M) * (l == 2 ? C : H)));
     RTE_CUDA(H1.alloc((size_t)M * H));
     RTE_CUDA(H2.alloc((size_t)M * H));
     RTE_CUDA(Z.alloc((size_t)M * C));
@@ -276,37 +276,82 @@ struct StepBufs {
   }
 };
 
+// Two more streams beside the caller's, for the parts of a step that do not
+// depend on one another.  The destructor waits for both, so that nothing they
+// use is freed under them on an early return.
+struct StepStreams {
+  cudaStream_t side[2] = {nullptr, nullptr};
+  cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
+  StepStreams() = default;
+  StepStreams(const StepStreams&) = delete;
+  rte_status create() {
+    for (cudaStream_t& s : side) RTE_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    for (cudaEvent_t& e : ev) RTE_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    return RTE_OK;
+  }
+  ~StepStreams() {
+    for (cudaStream_t s : side)
+      if (s) {
+        cudaStreamSynchronize(s);
+        cudaStreamDestroy(s);
+      }
+    for (cudaEvent_t e : ev)
+      if (e) cudaEventDestroy(e);
+  }
+  // `to` waits for all work recorded so far on `from`, through event e.
+  cudaError_t follow(cudaStream_t from, cudaStream_t to, int e) {
+    const cudaError_t r = cudaEventRecord(ev[e], from);
+    return r != cudaSuccess ? r : cudaStreamWaitEvent(to, ev[e], 0);
+  }
+};
+
 // Forward and backward of the MLP on one batch: Xb [M x dp] BF16, labels
 // yb [M]; writes the FP32 gradients gw[l] (same shapes as the weights) and
 // gb[l] and the per-row loss.  Mean cross-entropy over the batch.
+// With `ss` (its streams idle, or behind st), the weight transposes run beside
+// the forward pass, and each layer's weight and bias gradients beside the next
+// layer's input gradients: the gradient GEMMs have 2 to 64 tiles and K = M, so
+// alone they leave most of the GPU idle.  st has all results when it returns.
 rte_status fwd_bwd(const Mlp& m, const uint16_t* Xb, const int32_t* yb, int M, StepBufs& b,
-                   float* const gw[3], float* const gb[3], int* err, cudaStream_t st) {
+                   float* const gw[3], float* const gb[3], int* err, cudaStream_t st, StepStreams* ss = nullptr) {
   const int H = m.hidden, C = m.classes, dp = m.dp;
+  cudaStream_t s1 = ss ? ss->side[0] : st, s2 = ss ? ss->side[1] : st;
+  if (ss) RTE_CUDA(ss->follow(st, s1, 0));
+  RTE_CUDA(launch_transpose_bf16(m.W16[2].p, C, H, b.W3T.p, s1));
+  RTE_CUDA(launch_transpose_bf16(m.W16[1].p, H, H, b.W2T.p, s1));
+  RTE_CUDA(launch_transpose_bf16(Xb, M, dp, b.XT.p, s1));
   RTE_CUDA(gemm(Xb, m.W16[0].p, M, H, dp, kEpiBiasReluBF16, b.H1.p, H, m.b[0].p, nullptr, err, st));
+  if (ss) RTE_CUDA(ss->follow(st, s2, 1));
+  RTE_CUDA(launch_transpose_bf16(b.H1.p, M, H, b.H1T.p, s2));
   RTE_CUDA(gemm(b.H1.p, m.W16[1].p, M, H, H, kEpiBiasReluBF16, b.H2.p, H, m.b[1].p, nullptr, err, st));
+  if (ss) RTE_CUDA(ss->follow(st, s1, 2));
+  RTE_CUDA(launch_transpose_bf16(b.H2.p, M, H, b.H2T.p, s1));
+  if (ss) RTE_CUDA(cudaEventRecord(ss->ev[3], s1));  // W3T, W2T, XT and H2T are done
   RTE_CUDA(gemm(b.H2.p, m.W16[2].p, M, C, H, kEpiBiasF32, b.Z.p, C, m.b[2].p, nullptr, err, st));
   RTE_CUDA(launch_softmax_ce(b.Z.p, M, C, yb, 1.0f / M, b.dZ.p, b.loss.p, st));
   // layer 3: dW3 = dZ^T H2, db3 = colsum(dZ), dH2 = relu'(H2) * (dZ W3)
-  RTE_CUDA(launch_transpose_bf16(b.dZ.p, M, C, b.dZT.p, st));
-  RTE_CUDA(launch_transpose_bf16(b.H2.p, M, H, b.H2T.p, st));
-  RTE_CUDA(gemm(b.dZT.p, b.H2T.p, C, H, M, kEpiStoreF32, gw[2], H, nullptr, nullptr, err, st));
-  RTE_CUDA(launch_col_sum_bf16(b.dZ.p, M, C, gb[2], b.colpart.p, st));
-  RTE_CUDA(launch_transpose_bf16(m.W16[2].p, C, H, b.W3T.p, st));
+  if (ss) RTE_CUDA(ss->follow(st, s1, 0));
+  RTE_CUDA(launch_transpose_bf16(b.dZ.p, M, C, b.dZT.p, s1));
+  RTE_CUDA(gemm(b.dZT.p, b.H2T.p, C, H, M, kEpiStoreF32, gw[2], H, nullptr, nullptr, err, s1));
+  RTE_CUDA(launch_col_sum_bf16(b.dZ.p, M, C, gb[2], b.colpart[2].p, s1));
+  if (ss) RTE_CUDA(cudaStreamWaitEvent(st, ss->ev[3], 0));
   RTE_CUDA(gemm(b.dZ.p, b.W3T.p, M, H, C, kEpiStoreF32, b.dH2f.p, H, nullptr, nullptr, err, st));
   RTE_CUDA(launch_relu_grad(b.dH2f.p, b.H2.p, (int64_t)M * H, b.dH2.p, st));
   // layer 2
-  RTE_CUDA(launch_transpose_bf16(b.dH2.p, M, H, b.dH2T.p, st));
-  RTE_CUDA(launch_transpose_bf16(b.H1.p, M, H, b.H1T.p, st));
-  RTE_CUDA(gemm(b.dH2T.p, b.H1T.p, H, H, M, kEpiStoreF32, gw[1], H, nullptr, nullptr, err, st));
-  RTE_CUDA(launch_col_sum_bf16(b.dH2.p, M, H, gb[1], b.colpart.p, st));
-  RTE_CUDA(launch_transpose_bf16(m.W16[1].p, H, H, b.W2T.p, st));
+  if (ss) RTE_CUDA(ss->follow(st, s2, 1));
+  RTE_CUDA(launch_transpose_bf16(b.dH2.p, M, H, b.dH2T.p, s2));
+  RTE_CUDA(gemm(b.dH2T.p, b.H1T.p, H, H, M, kEpiStoreF32, gw[1], H, nullptr, nullptr, err, s2));
+  RTE_CUDA(launch_col_sum_bf16(b.dH2.p, M, H, gb[1], b.colpart[1].p, s2));
   RTE_CUDA(gemm(b.dH2.p, b.W2T.p, M, H, H, kEpiStoreF32, b.dH1f.p, H, nullptr, nullptr, err, st));
   RTE_CUDA(launch_relu_grad(b.dH1f.p, b.H1.p, (int64_t)M * H, b.dH1.p, st));
   // layer 1
   RTE_CUDA(launch_transpose_bf16(b.dH1.p, M, H, b.dH1T.p, st));
-  RTE_CUDA(launch_transpose_bf16(Xb, M, dp, b.XT.p, st));
   RTE_CUDA(gemm(b.dH1T.p, b.XT.p, H, dp, M, kEpiStoreF32, gw[0], dp, nullptr, nullptr, err, st));
-  RTE_CUDA(launch_col_sum_bf16(b.dH1.p, M, H, gb[0], b.colpart.p, st));
+  RTE_CUDA(launch_col_sum_bf16(b.dH1.p, M, H, gb[0], b.colpart[0].p, st));
+  if (ss) {
+    RTE_CUDA(ss->follow(s1, st, 2));
+    RTE_CUDA(ss->follow(s2, st, 1));
+  }
   return RTE_OK;
 }
 
@@ -446,34 +491,28 @@ extern "C" rte_status rte_learned_train(rte_index* x, const float* train_queries
   } else {
     RTE_CUDA(cudaMemcpy(proj.p, q32.p, proj.bytes(), cudaMemcpyDeviceToDevice));
   }
-  q32.reset();
-  // 2. labels: leaf of the plain search's best result
-  DevBuf<int32_t> top;
-  RTE_CUDA(top.alloc(n));
-  rte_status s = plain_top1(x, proj.p, n, tp->label_beam, top.p, st);
-  if (s != RTE_OK) return s;
-  std::vector<int32_t> ids(n), leaf_of(x->np, 0), labels(n);
-  RTE_CUDA(cudaMemcpy(ids.data(), top.p, n * 4, cudaMemcpyDeviceToHost));
-  for (int64_t l = 0; l < x->kd.n_leaves; ++l)
-    for (int j = 0; j < x->kd.cap; ++j) {
-      const int32_t p = x->kd.pids[l * x->kd.cap + j];
-      if (p < x->np) leaf_of[p] = (int32_t)l;
-    }
-  for (int64_t i = 0; i < n; ++i)
-    labels[i] = leaf_class[(ids[i] >= 0 && ids[i] < x->np) ? leaf_of[ids[i]] : 0];
-  DevBuf<int32_t> d_labels;
-  RTE_CUDA(d_labels.alloc(n));
-  RTE_CUDA(cudaMemcpy(d_labels.p, labels.data(), n * 4, cudaMemcpyHostToDevice));
-  // 3. inputs: BF16 of the projected query scaled to unit RMS
+  // the input scale needs the first projected queries on the host; what
+  // follows on the host runs beside the labelling search
   std::vector<float> sample((size_t)std::min<int64_t>(n, 4096) * d);
   RTE_CUDA(cudaMemcpy(sample.data(), proj.p, sample.size() * 4, cudaMemcpyDeviceToHost));
+  // 2. labels: class of the leaf of the plain search's best result
+  DevBuf<int32_t> top, d_labels, d_leaf_class, point_class;
+  RTE_CUDA(top.alloc(n));
+  RTE_CUDA(d_labels.alloc(n));
+  RTE_CUDA(d_leaf_class.alloc(leaf_class.size()));
+  RTE_CUDA(point_class.alloc(x->np));
+  RTE_CUDA(cudaMemcpy(d_leaf_class.p, leaf_class.data(), leaf_class.size() * 4, cudaMemcpyHostToDevice));
+  DevBuf<uint16_t> X;
+  RTE_CUDA(X.alloc((size_t)n * dp));
+  rte_status s = plain_top1(x, proj.p, n, tp->label_beam, top.p, st);
+  if (s != RTE_OK) return s;
+  RTE_CUDA(launch_point_labels(top.p, n, x->d_pids.p, x->kd.n_leaves, x->kd.cap, x->np, d_leaf_class.p,
+                               point_class.p, d_labels.p, st));
+  // 3. inputs: BF16 of the projected query scaled to unit RMS
   double ss = 0;
   for (float v : sample) ss += (double)v * v;
   const float in_scale = (float)(1.0 / std::sqrt(std::max(ss / sample.size(), 1e-30)));
-  DevBuf<uint16_t> X;
-  RTE_CUDA(X.alloc((size_t)n * dp));
   RTE_CUDA(launch_cast_rows_bf16(proj.p, n, d, d, in_scale, dp, X.p, st));
-  proj.reset();
   // 4. parameters (He-uniform, fixed seed), Adam moments
   Mlp m;
   m.d_in = d;
@@ -490,8 +529,11 @@ extern "C" rte_status rte_learned_train(rte_index* x, const float* train_queries
   const int fan[3] = {d, H, H};
   DevBuf<float> mw[3], vw[3], mb[3], vb[3], gw[3], gb[3];
   std::mt19937 rng((uint32_t)tp->seed);
+  // every random number of the first epoch while the search runs
+  std::vector<float> hw[3], hb[3];
   for (int l = 0; l < 3; ++l) {
-    std::vector<float> w(wn[l]);
+    std::vector<float>& w = hw[l];
+    w.resize(wn[l]);
     const float lim = std::sqrt(6.0f / fan[l]);
     std::uniform_real_distribution<float> U(-lim, lim);
     for (int64_t i = 0; i < wn[l]; ++i) w[i] = U(rng);
@@ -500,23 +542,19 @@ extern "C" rte_status rte_learned_train(rte_index* x, const float* train_queries
         for (int c = d; c < dp; ++c) w[(int64_t)r * dp + c] = 0.f;
     if (l == 2)  // padded classes: zero weights
       for (int64_t i = C * H; i < Cp * H; ++i) w[i] = 0.f;
-    std::vector<float> bias(bn[l], 0.f);
+    hb[l].assign(bn[l], 0.f);
     if (l == 2)
-      for (int64_t i = C; i < Cp; ++i) bias[i] = -1e30f;
+      for (int64_t i = C; i < Cp; ++i) hb[l][i] = -1e30f;
+  }
+  std::vector<int64_t> order(n);
+  for (int64_t i = 0; i < n; ++i) order[i] = i;
+  std::shuffle(order.begin(), order.end(), rng);
+  for (int l = 0; l < 3; ++l) {
     RTE_CUDA(m.W[l].alloc(wn[l]));
     RTE_CUDA(m.W16[l].alloc(wn[l]));
     RTE_CUDA(m.b[l].alloc(bn[l]));
-    RTE_CUDA(cudaMemcpy(m.W[l].p, w.data(), wn[l] * 4, cudaMemcpyHostToDevice));
-    RTE_CUDA(cudaMemcpy(m.b[l].p, bias.data(), bn[l] * 4, cudaMemcpyHostToDevice));
-    RTE_CUDA(launch_f32_to_bf16(m.W[l].p, wn[l], m.W16[l].p, st));
-    for (DevBuf<float>* b : {&mw[l], &vw[l], &gw[l]}) {
-      RTE_CUDA(b->alloc(wn[l]));
-      RTE_CUDA(cudaMemset(b->p, 0, b->bytes()));
-    }
-    for (DevBuf<float>* b : {&mb[l], &vb[l], &gb[l]}) {
-      RTE_CUDA(b->alloc(bn[l]));
-      RTE_CUDA(cudaMemset(b->p, 0, b->bytes()));
-    }
+    for (DevBuf<float>* b : {&mw[l], &vw[l], &gw[l]}) RTE_CUDA(b->alloc(wn[l]));
+    for (DevBuf<float>* b : {&mb[l], &vb[l], &gb[l]}) RTE_CUDA(b->alloc(bn[l]));
   }
   // 5. per-batch buffers
   StepBufs sb;
@@ -530,11 +568,19 @@ extern "C" rte_status rte_learned_train(rte_index* x, const float* train_queries
   RTE_CUDA(yb.alloc(M));
   RTE_CUDA(perm.alloc(n));
   RTE_CUDA(err.alloc(1));
+  StepStreams streams;
+  s = streams.create();
+  if (s != RTE_OK) return s;
   RTE_CUDA(cudaMemset(err.p, 0, 4));
+  for (int l = 0; l < 3; ++l) {
+    RTE_CUDA(cudaMemcpy(m.W[l].p, hw[l].data(), wn[l] * 4, cudaMemcpyHostToDevice));
+    RTE_CUDA(cudaMemcpy(m.b[l].p, hb[l].data(), bn[l] * 4, cudaMemcpyHostToDevice));
+    RTE_CUDA(launch_f32_to_bf16(m.W[l].p, wn[l], m.W16[l].p, st));
+    for (DevBuf<float>* b : {&mw[l], &vw[l], &gw[l], &mb[l], &vb[l], &gb[l]})
+      RTE_CUDA(cudaMemsetAsync(b->p, 0, b->bytes(), st));
+  }
   float* const gwp[3] = {gw[0].p, gw[1].p, gw[2].p};
   float* const gbp[3] = {gb[0].p, gb[1].p, gb[2].p};
-  std::vector<int64_t> order(n);
-  for (int64_t i = 0; i < n; ++i) order[i] = i;
   const int64_t steps_per_epoch = n / M;
   const int64_t total = steps_per_epoch * tp->epochs;
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
@@ -546,23 +592,29 @@ extern "C" rte_status rte_learned_train(rte_index* x, const float* train_queries
   cudaEventCreate(&e1);
   cudaEventRecord(e0, st);
   for (int ep = 0; ep < tp->epochs; ++ep) {
-    std::shuffle(order.begin(), order.end(), rng);
+    if (ep > 0) std::shuffle(order.begin(), order.end(), rng);
     RTE_CUDA(cudaMemcpy(perm.p, order.data(), n * 8, cudaMemcpyHostToDevice));
     for (int64_t sidx = 0; sidx < steps_per_epoch; ++sidx, ++t) {
       RTE_CUDA(launch_gather_rows(X.p, dp, perm.p + sidx * M, M, d_labels.p, Xb.p, yb.p, st));
-      s = fwd_bwd(m, Xb.p, yb.p, M, sb, gwp, gbp, err.p, st);
+      s = fwd_bwd(m, Xb.p, yb.p, M, sb, gwp, gbp, err.p, st, &streams);
       if (s != RTE_OK) return s;
       // Adam with a cosine decay to a tenth of the rate
       const float frac = total > 1 ? (float)t / (float)(total - 1) : 0.f;
       const float lr = tp->lr * (0.1f + 0.9f * 0.5f * (1.f + std::cos(3.14159265f * frac)));
       const float c1 = 1.f / (1.f - std::pow(b1, (float)(t + 1)));
       const float c2 = 1.f / (1.f - std::pow(b2, (float)(t + 1)));
+      AdamArgs ad{};
       for (int l = 0; l < 3; ++l) {
-        RTE_CUDA(launch_adam(m.W[l].p, gw[l].p, mw[l].p, vw[l].p, wn[l], lr, b1, b2, eps, c1, c2,
-                             m.W16[l].p, st));
-        RTE_CUDA(launch_adam(m.b[l].p, gb[l].p, mb[l].p, vb[l].p, bn[l], lr, b1, b2, eps, c1, c2,
-                             nullptr, st));
+        ad.t[2 * l] = AdamTensor{m.W[l].p, gw[l].p, mw[l].p, vw[l].p, m.W16[l].p, wn[l], 0};
+        ad.t[2 * l + 1] = AdamTensor{m.b[l].p, gb[l].p, mb[l].p, vb[l].p, nullptr, bn[l], 0};
       }
+      ad.lr = lr;
+      ad.b1 = b1;
+      ad.b2 = b2;
+      ad.eps = eps;
+      ad.c1 = c1;
+      ad.c2 = c2;
+      RTE_CUDA(launch_adam(ad, st));
       if (t == 0 || t == total - 1) {
         RTE_CUDA(cudaMemcpy(hl.data(), sb.loss.p, M * 4, cudaMemcpyDeviceToHost));
         double sl = 0;

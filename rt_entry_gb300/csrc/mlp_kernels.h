@@ -16,9 +16,28 @@ cudaError_t launch_relu_grad(const float* g, const void* h, int64_t n, void* out
 constexpr int kColSumMaxSlices = 64;
 int col_sum_slices(int M);
 cudaError_t launch_col_sum_bf16(const void* x, int M, int N, float* out, float* part, cudaStream_t st);
-cudaError_t launch_adam(float* w, const float* g, float* m1, float* m2, int64_t n, float lr,
-                        float b1, float b2, float eps, float c1, float c2, void* w16,
-                        cudaStream_t st);
+// One Adam step on every parameter tensor (weights and biases of the three
+// layers) in one launch.
+constexpr int kAdamTensors = 6;
+struct AdamTensor {
+  float* w;
+  const float* g;
+  float* m1;
+  float* m2;
+  void* w16;  // BF16 copy, or null
+  int64_t n;
+  int first;  // first block (set by launch_adam)
+};
+struct AdamArgs {
+  AdamTensor t[kAdamTensors];
+  float lr, b1, b2, eps, c1, c2;
+};
+cudaError_t launch_adam(AdamArgs a, cudaStream_t st);
+// labels[i]: the class of base point ids[i], which is that of the kd-tree leaf
+// (class_of_leaf) listing it in pids [n_leaves][cap]; point_class: scratch [np].
+cudaError_t launch_point_labels(const int32_t* ids, int64_t n, const int32_t* pids, int64_t n_leaves, int cap,
+                                int64_t np, const int32_t* class_of_leaf, int32_t* point_class, int32_t* labels,
+                                cudaStream_t st);
 cudaError_t launch_f32_to_bf16(const float* x, int64_t n, void* out, cudaStream_t st);
 cudaError_t launch_gather_rows(const void* src, int dp, const int64_t* idx, int rows,
                                const int32_t* labels_src, void* dst, int32_t* labels_dst,
