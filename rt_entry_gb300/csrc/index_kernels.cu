@@ -21,19 +21,33 @@
 
 #include "index_kernels.h"
 #include "layout.cuh"
+#include "widen.cuh"
 
 namespace rte {
 
 // ---------------------------------------------------------------- mean ----
 // Block b sums rows [b*rows_per_block, ...) of every column in FP64 into
-// partial[b][col]; a second kernel adds the partials in block order.
+// partial[b][col]; a second kernel adds the partials in block order.  Both
+// add one value at a time (the order is the result); kMeanAhead loads are in
+// flight ahead of the sums.  300k x 128 on one GB300: 163 + 127 us without
+// them, 162 + 79 us with.
+constexpr int kMeanAhead = 16;
+
 __global__ void col_sum_partial(const float* __restrict__ x, int64_t n, int d,
                                 int64_t rows_per_block, double* __restrict__ partial) {
   const int64_t r0 = (int64_t)blockIdx.x * rows_per_block;
   const int64_t r1 = min(n, r0 + rows_per_block);
   for (int c = threadIdx.x; c < d; c += blockDim.x) {
     double s = 0.0;
-    for (int64_t r = r0; r < r1; ++r) s += (double)x[r * d + c];
+    int64_t r = r0;
+    for (; r + kMeanAhead <= r1; r += kMeanAhead) {
+      float v[kMeanAhead];
+#pragma unroll
+      for (int u = 0; u < kMeanAhead; ++u) v[u] = __ldg(x + (r + u) * d + c);
+#pragma unroll
+      for (int u = 0; u < kMeanAhead; ++u) s += widen(v[u]);
+    }
+    for (; r < r1; ++r) s += (double)x[r * d + c];
     partial[(int64_t)blockIdx.x * d + c] = s;
   }
 }
@@ -43,42 +57,93 @@ __global__ void col_sum_finish(const double* __restrict__ partial, int nblocks, 
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= d) return;
   double s = 0.0;
-  for (int b = 0; b < nblocks; ++b) s += partial[(int64_t)b * d + c];
+  double v[2][kMeanAhead];
+  auto load = [&](double (&w)[kMeanAhead], int b) {
+#pragma unroll
+    for (int u = 0; u < kMeanAhead; ++u) w[u] = b + u < nblocks ? __ldg(partial + (int64_t)(b + u) * d + c) : 0.0;
+  };
+  auto add = [&](const double (&w)[kMeanAhead], int b) {
+#pragma unroll
+    for (int u = 0; u < kMeanAhead; ++u)
+      if (b + u < nblocks) s += w[u];
+  };
+  load(v[0], 0);
+  for (int b = 0; b < nblocks; b += 2 * kMeanAhead) {
+    load(v[1], b + kMeanAhead);
+    add(v[0], b);
+    load(v[0], b + 2 * kMeanAhead);
+    add(v[1], b + kMeanAhead);
+  }
   mean[c] = s / (double)n;
 }
 
 // ---------------------------------------------------------- covariance ----
-// Tile of 32x32 outputs per block (16x16 threads, 2x2 each) over a chunk of
-// rows; rows are centred in FP64 as they are staged in shared memory.
-constexpr int kCovTile = 32;
+// The covariance is symmetric, and (i, j) and (j, i) sum the same products in
+// the same order, so only tiles that reach the diagonal or lie above it are
+// computed and cov_finish mirrors them.  FP64 bounds this (1.25 TFLOP/s on a
+// GB300): a block of 128 threads (2 x 2 outputs each) computes a tile of 16 x
+// 32, small enough that 20 of 32 tiles do at d = 128 and that the chunks'
+// blocks spread evenly over the SMs, over a chunk of rows; rows are centred
+// in FP64 as they are staged in shared memory.  300k x 128: 9.5 ms for all
+// tiles of 32 x 32, 6.6 ms now.
+constexpr int kCovRows = 16;
+constexpr int kCovCols = 32;
 constexpr int kCovK = 32;
+constexpr int kCovThreads = 128;
 
-__global__ void cov_partial(const float* __restrict__ x, int64_t n, int d,
+__global__ void __launch_bounds__(kCovThreads) cov_partial(const float* __restrict__ x, int64_t n, int d,
                             const double* __restrict__ mean, int64_t rows_per_chunk,
                             double* __restrict__ partial) {
-  __shared__ double sa[kCovK][kCovTile + 1];
-  __shared__ double sb[kCovK][kCovTile + 1];
-  const int i0 = blockIdx.y * kCovTile, j0 = blockIdx.x * kCovTile;
-  const int64_t r0 = (int64_t)blockIdx.z * rows_per_chunk;
+  __shared__ double sa[kCovK][kCovRows + 1];
+  __shared__ double sb[kCovK][kCovCols + 1];
+  // block x: the x-th tile, row by row, of those not below the diagonal (an
+  // idle block for each of the others would leave the SMs with 5 to 13 busy
+  // ones each: all are resident at once)
+  int ta = 0, tb = blockIdx.x;
+  for (; tb >= (d + kCovCols - 1) / kCovCols - ta * kCovRows / kCovCols; ++ta)
+    tb -= (d + kCovCols - 1) / kCovCols - ta * kCovRows / kCovCols;
+  tb += ta * kCovRows / kCovCols;
+  const int i0 = ta * kCovRows, j0 = tb * kCovCols;
+  const int64_t r0 = (int64_t)blockIdx.y * rows_per_chunk;
   const int64_t r1 = min(n, r0 + rows_per_chunk);
-  const int tx = threadIdx.x, ty = threadIdx.y;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   double acc[2][2] = {{0, 0}, {0, 0}};
+  // this thread stages one column of each operand
+  const int ca = threadIdx.x & (kCovRows - 1), ra = threadIdx.x / kCovRows;
+  const int cb = threadIdx.x & (kCovCols - 1), rb0 = threadIdx.x / kCovCols;
+  const bool ina = i0 + ca < d, inb = j0 + cb < d;
+  const double ma = ina ? mean[i0 + ca] : 0.0, mb = inb ? mean[j0 + cb] : 0.0;
+  constexpr int kLoadA = kCovK * kCovRows / kCovThreads, kLoadB = kCovK * kCovCols / kCovThreads;
+  float va[kLoadA], vb[kLoadB];
+  auto load = [&](int64_t rb) {
+#pragma unroll
+    for (int u = 0; u < kLoadA; ++u) {
+      const int64_t r = rb + ra + u * (kCovThreads / kCovRows);
+      va[u] = r < r1 && ina ? __ldg(x + r * d + i0 + ca) : 0.0f;
+    }
+#pragma unroll
+    for (int u = 0; u < kLoadB; ++u) {
+      const int64_t r = rb + rb0 + u * (kCovThreads / kCovCols);
+      vb[u] = r < r1 && inb ? __ldg(x + r * d + j0 + cb) : 0.0f;
+    }
+  };
+  load(r0);
   for (int64_t rb = r0; rb < r1; rb += kCovK) {
-    for (int t = ty * 16 + tx; t < kCovK * kCovTile; t += 256) {
-      const int rr = t / kCovTile, cc = t % kCovTile;
-      const int64_t r = rb + rr;
-      double va = 0.0, vb = 0.0;
-      if (r < r1) {
-        if (i0 + cc < d) va = (double)x[r * d + i0 + cc] - mean[i0 + cc];
-        if (j0 + cc < d) vb = (double)x[r * d + j0 + cc] - mean[j0 + cc];
-      }
-      sa[rr][cc] = va;
-      sb[rr][cc] = vb;
+#pragma unroll
+    for (int u = 0; u < kLoadA; ++u) {
+      const int rr = ra + u * (kCovThreads / kCovRows);
+      sa[rr][ca] = rb + rr < r1 && ina ? widen(va[u]) - ma : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < kLoadB; ++u) {
+      const int rr = rb0 + u * (kCovThreads / kCovCols);
+      sb[rr][cb] = rb + rr < r1 && inb ? widen(vb[u]) - mb : 0.0;
     }
     __syncthreads();
+    if (rb + kCovK < r1) load(rb + kCovK);  // in flight during the products
 #pragma unroll 4
     for (int k = 0; k < kCovK; ++k) {
-      const double a0 = sa[k][ty], a1 = sa[k][ty + 16];
+      const double a0 = sa[k][ty], a1 = sa[k][ty + 8];
       const double b0 = sb[k][tx], b1 = sb[k][tx + 16];
       acc[0][0] = fma(a0, b0, acc[0][0]);
       acc[0][1] = fma(a0, b1, acc[0][1]);
@@ -87,10 +152,10 @@ __global__ void cov_partial(const float* __restrict__ x, int64_t n, int d,
     }
     __syncthreads();
   }
-  double* out = partial + (int64_t)blockIdx.z * d * d;
+  double* out = partial + (int64_t)blockIdx.y * d * d;
   for (int a = 0; a < 2; ++a)
     for (int b = 0; b < 2; ++b) {
-      const int i = i0 + ty + 16 * a, j = j0 + tx + 16 * b;
+      const int i = i0 + ty + 8 * a, j = j0 + tx + 16 * b;
       if (i < d && j < d) out[(int64_t)i * d + j] = acc[a][b];
     }
 }
@@ -100,8 +165,11 @@ __global__ void cov_finish(const double* __restrict__ partial, int nchunks, int 
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t dd = (int64_t)d * d;
   if (e >= dd) return;
+  const int64_t i = e / d, j = e - i * d;
+  const int64_t u = i <= j ? e : j * d + i;  // the computed one of (i, j) and (j, i)
   double s = 0.0;
-  for (int c = 0; c < nchunks; ++c) s += partial[c * dd + e];
+#pragma unroll 8
+  for (int c = 0; c < nchunks; ++c) s += __ldg(partial + c * dd + u);
   cov[e] = s / (double)(n - 1);
 }
 
@@ -591,15 +659,16 @@ cudaError_t launch_mean(const float* x, int64_t n, int d, double* partial, int n
                         double* mean, cudaStream_t st) {
   const int64_t rpb = (n + nblocks - 1) / nblocks;
   col_sum_partial<<<nblocks, 128, 0, st>>>(x, n, d, rpb, partial);
-  col_sum_finish<<<(d + 127) / 128, 128, 0, st>>>(partial, nblocks, d, n, mean);
+  col_sum_finish<<<(d + 31) / 32, 32, 0, st>>>(partial, nblocks, d, n, mean);
   return cudaGetLastError();
 }
 
 cudaError_t launch_cov(const float* x, int64_t n, int d, const double* mean, double* partial,
                        int nchunks, double* cov, cudaStream_t st) {
   const int64_t rpc = (n + nchunks - 1) / nchunks;
-  dim3 grid((d + kCovTile - 1) / kCovTile, (d + kCovTile - 1) / kCovTile, nchunks);
-  cov_partial<<<grid, dim3(16, 16), 0, st>>>(x, n, d, mean, rpc, partial);
+  int tiles = 0;
+  for (int i0 = 0; i0 < d; i0 += kCovRows) tiles += (d + kCovCols - 1) / kCovCols - i0 / kCovCols;
+  cov_partial<<<dim3(tiles, nchunks), kCovThreads, 0, st>>>(x, n, d, mean, rpc, partial);
   const int64_t dd = (int64_t)d * d;
   cov_finish<<<(unsigned)((dd + 255) / 256), 256, 0, st>>>(partial, nchunks, d, n, cov);
   return cudaGetLastError();

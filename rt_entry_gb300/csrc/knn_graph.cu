@@ -47,6 +47,7 @@
 #include "knn_filter.h"
 #include "index_impl.h"
 #include "rtentry.h"
+#include "widen.cuh"
 
 namespace rte {
 namespace {
@@ -355,17 +356,6 @@ __global__ void __launch_bounds__(256) sample_threshold(const float* __restrict_
     if (__reduce_add_sync(0xffffffffu, below) < (unsigned)rank) at |= bit;
   }
   if (lane == 0) tau[row] = key_float(at);
-}
-
-// FP32 -> FP64 with integer instructions: the conversion instruction runs at
-// the FP64 unit's rate, a sixty-fourth of theirs, and there would be two for
-// every two FP64 operations.  Exact for zeros and normal numbers; `special`
-// is set for the rest (denormals, infinities, NaN).
-__device__ __forceinline__ double widen(float f, bool& special) {
-  const uint32_t u = __float_as_uint(f), e = u & 0x7f800000u;
-  special |= e == 0x7f800000u || (e == 0u && (u & 0x007fffffu) != 0u);
-  const uint32_t hi = e == 0u ? u : (u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u);
-  return __hiloint2double((int)hi, (int)(u << 29));
 }
 
 // Step 3: one warp per row and eight rows per block.  The R-th smallest
