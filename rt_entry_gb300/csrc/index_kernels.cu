@@ -21,6 +21,7 @@
 
 #include "index_kernels.h"
 #include "layout.cuh"
+#include "pdl.cuh"
 #include "widen.cuh"
 
 namespace rte {
@@ -488,6 +489,8 @@ __global__ void locate_points(const WideNode* __restrict__ wide, int n_wide,
                               const float* __restrict__ pts, int64_t n, int stride,
                               int32_t* __restrict__ out, const int* __restrict__ n_dev) {
   __shared__ WideNode top[kTop ? kTopWide : 1];
+  dependency_wait();
+  allow_dependents();
   if (n_dev) n = min(n, (int64_t)*n_dev);
   if ((int64_t)blockIdx.x * blockDim.x >= n) return;
   prefetch_tree(wide, n_wide);
@@ -559,6 +562,8 @@ __global__ void locate_in_subtree_wide(const WideNode* __restrict__ wide,
                                        const int32_t* __restrict__ start_ref,
                                        const int32_t* __restrict__ fallback_leaf, int n_classes,
                                        const int* __restrict__ n_dev, int32_t* __restrict__ out) {
+  dependency_wait();
+  allow_dependents();
   if (n_dev) n = min(n, (int64_t)*n_dev);  // graph replay: points beyond the batch are idle
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -785,10 +790,9 @@ cudaError_t launch_locate_in_subtree_wide(const WideNode* wide, const float* pts
                                           int n_classes, int32_t* out, cudaStream_t st,
                                           const int* n_dev) {
   if (n == 0) return cudaSuccess;
-  locate_in_subtree_wide<<<(unsigned)((n + 63) / 64), 64, 0, st>>>(wide, pts, n, stride, keys,
-                                                                     start_ref, fallback_leaf, n_classes,
-                                                                     n_dev, out);
-  return cudaGetLastError();
+  void* args[] = {&wide, &pts, &n, &stride, &keys, &start_ref, &fallback_leaf, &n_classes, &n_dev, &out};
+  return launch_pdl((const void*)locate_in_subtree_wide, dim3((unsigned)((n + 63) / 64)), dim3(64), 0, st, args, n,
+                    n_dev);
 }
 
 cudaError_t launch_locate_multi(const WideNode* wide, int n_wide, const float* pts, int64_t n,
@@ -801,20 +805,14 @@ cudaError_t launch_locate_multi(const WideNode* wide, int n_wide, const float* p
 cudaError_t launch_locate(const WideNode* wide, int n_wide, const float* pts, int64_t n, int stride,
                           int32_t* out, cudaStream_t st, bool top_cache) {
   if (n == 0) return cudaSuccess;
-  if (top_cache)
-    locate_points<true><<<(unsigned)((n + 63) / 64), 64, 0, st>>>(wide, n_wide, pts, n, stride, out, nullptr);
-  else
-    locate_points<false><<<(unsigned)((n + 63) / 64), 64, 0, st>>>(wide, n_wide, pts, n, stride, out, nullptr);
-  return cudaGetLastError();
+  return launch_locate_dyn(wide, n_wide, pts, n, nullptr, stride, out, st, top_cache);
 }
 
 cudaError_t launch_locate_dyn(const WideNode* wide, int n_wide, const float* pts, int64_t cap,
                               const int* n_dev, int stride, int32_t* out, cudaStream_t st, bool top_cache) {
-  if (top_cache)
-    locate_points<true><<<(unsigned)((cap + 63) / 64), 64, 0, st>>>(wide, n_wide, pts, cap, stride, out, n_dev);
-  else
-    locate_points<false><<<(unsigned)((cap + 63) / 64), 64, 0, st>>>(wide, n_wide, pts, cap, stride, out, n_dev);
-  return cudaGetLastError();
+  void* args[] = {&wide, &n_wide, &pts, &cap, &stride, &out, &n_dev};
+  return launch_pdl(top_cache ? (const void*)locate_points<true> : (const void*)locate_points<false>,
+                    dim3((unsigned)((cap + 63) / 64)), dim3(64), 0, st, args, cap, n_dev);
 }
 
 // Counting sort of the queries by leaf range: count per range, exclusive
@@ -837,6 +835,8 @@ __global__ void __launch_bounds__(kOrderThreads) order_by_leaf_kernel(const int3
                                                                       const int* n_dev, int64_t min_n) {
   __shared__ int cnt[kOrderBins];
   __shared__ int wsum[kOrderThreads / 32];
+  dependency_wait();
+  allow_dependents();
   if (n_dev) {  // the live count, at most the capacity n
     const int64_t live = *n_dev;
     n = live < 0 ? 0 : live < n ? live : n;
@@ -914,8 +914,8 @@ cudaError_t launch_order_by_leaf(const int32_t* leaf, int stride, int64_t n, int
   if (n > INT32_MAX || n_leaves < 1 || stride < 1) return cudaErrorInvalidValue;
   int shift = 0;
   while (((n_leaves - 1) >> shift) >= kOrderBins) ++shift;
-  order_by_leaf_kernel<<<1, kOrderThreads, 0, st>>>(leaf, stride, n, n_leaves, shift, order, n_dev, min_n);
-  return cudaGetLastError();
+  void* args[] = {&leaf, &stride, &n, &n_leaves, &shift, &order, &n_dev, &min_n};
+  return launch_pdl((const void*)order_by_leaf_kernel, dim3(1), dim3(kOrderThreads), 0, st, args, n, n_dev);
 }
 
 }  // namespace rte

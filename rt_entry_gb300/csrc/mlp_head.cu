@@ -31,6 +31,7 @@
 
 #include "gemm_tc.h"
 #include "mlp_head.h"
+#include "pdl.cuh"
 #include "tc_common.cuh"
 
 namespace rte {
@@ -78,6 +79,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 8);
   __shared__ int s_abort;
 
+  dependency_wait();
+  allow_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int H = g.H;
   const int M = g.M_dev ? min(g.M, max(*g.M_dev, 0)) : g.M;  // rows of this launch
@@ -413,11 +416,9 @@ cudaError_t mlp_head_argmax(const MlpHeadArgs& a, cudaStream_t st) {
   const dim3 grid((unsigned)(tiles < sms ? tiles : sms));
   MlpHeadArgs ha = a;
   ha.wait_limit = wait_limit();
-  if (wide)
-    mlp_head_kernel<256><<<grid, kThreads, kSmemBytes, st>>>(mx, m1, m2, m3, ha);
-  else
-    mlp_head_kernel<128><<<grid, kThreads, kSmemBytes, st>>>(mx, m1, m2, m3, ha);
-  return cudaGetLastError();
+  void* args[] = {&mx, &m1, &m2, &m3, &ha};
+  return launch_pdl(wide ? (const void*)mlp_head_kernel<256> : (const void*)mlp_head_kernel<128>, grid, dim3(kThreads),
+                    kSmemBytes, st, args, ha.M, ha.M_dev);
 }
 
 }  // namespace rte

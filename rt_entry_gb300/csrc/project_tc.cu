@@ -41,6 +41,7 @@
 #include <atomic>
 #include <mutex>
 
+#include "pdl.cuh"
 #include "index_kernels.h"
 #include "tc_common.cuh"
 
@@ -90,6 +91,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     project_tf32_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmVh,
                         const __grid_constant__ CUtensorMap tmVl, ProjTcArgs p) {
   extern __shared__ uint8_t smem_raw[];
+  allow_dependents();
   if (p.zero) {  // a query call's counters and keys, zeroed on the way
     const int64_t nt = (int64_t)gridDim.x * blockDim.x;
     for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < p.zero_words; w += nt) p.zero[w] = 0u;

@@ -1,6 +1,8 @@
 // search_dispatch.cu -- maps (chunks, precision) to the instantiation files.
 #include "search_dispatch.h"
 
+#include "pdl.cuh"
+
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -114,6 +116,9 @@ cudaError_t launch_search(const SearchArgs& a, int C, int NL, int NB, int prec, 
   const size_t row = 32 * (size_t)C * (prec == kPrecF32 ? 4 : prec == kPrecBF16 ? 2 : 1);
   args.prefetch = row * (size_t)a.np > kL2ResidentRows;
   void* params[] = {&args};
+  // the team kernels serve the small batches; the single-warp ones begin
+  // without a dependency wait and are launched plainly
+  if (a.team != 0 && a.team != 1) return launch_pdl(k, dim3(grid), dim3(32 * wpb), smem, st, params, a.nq, a.nq_dev);
   return cudaLaunchKernel(k, dim3(grid), dim3(32 * wpb), params, smem, st);
 }
 

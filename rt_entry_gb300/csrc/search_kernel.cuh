@@ -5,10 +5,13 @@
 // one warp per query:
 //   * the pool (L = 32*NL slots, or 16 slots for NL = 0) and the batch
 //     (B = 32*NB slots) live in registers: slot p sits in lane p%32,
-//     register p/32.  The reference's
-//     comparator network (bitonic batch sort, pool/batch merge, half-cleaner,
-//     graph_search.cuh:888-957 and :1424-1493) runs on those registers,
-//     across lanes through shuffles and inside a lane for distances >= 32;
+//     register p/32.  The few candidates of a batch are compacted in shared
+//     memory and inserted or placed by rank, which gives the reference's
+//     result whenever no distances are equal; ties, NaN and larger counts
+//     run its comparator network (bitonic batch sort, pool/batch merge,
+//     half-cleaner, graph_search.cuh:888-957 and :1424-1493) on those
+//     registers, across lanes through shuffles and inside a lane for
+//     distances >= 32;
 //   * base rows are stored lane-interleaved (see layout.cuh): one 128-bit
 //     load gives lane l the dims l, l+32, l+64, l+96 -- exactly the dims the
 //     reference's reduction tree assigns to lane l -- so a neighbour row is a
@@ -32,6 +35,7 @@
 #include <type_traits>
 
 #include "layout.cuh"
+#include "pdl.cuh"
 #include "search_types.h"
 
 namespace rte {
@@ -1952,6 +1956,7 @@ __global__ void __launch_bounds__(256, search_min_blocks(C, NL, NB)) search_kern
 template <int C, int NL, int NB, int PREC, bool R16 = false>
 __global__ void __launch_bounds__(256, search_min_blocks(C, NL, NB)) search_kernel_team(SearchArgs a) {
   extern __shared__ uint32_t smem[];
+  dependency_wait();
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
   constexpr int B = batch_slots(NB);

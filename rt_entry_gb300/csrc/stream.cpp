@@ -8,7 +8,8 @@
 // search) captured once into a CUDA graph for batches of up to max_nq
 // queries.  The kernels read the batch size from device memory, so one
 // instantiated graph serves every batch size without re-capture; a batch
-// costs one graph launch plus the copies of its queries and results.  With
+// costs one graph launch plus the copy of its queries (and of its results
+// where the search cannot write them in place).  With
 // learned entries the graph holds the same five kernels as rte_search's
 // learned path: the projection (with the head's BF16 input and the zeroed
 // keys / counters), the fused head and the subtree location on the main
