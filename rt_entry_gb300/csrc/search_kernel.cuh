@@ -7,8 +7,8 @@
 //     (B = 32*NB slots) live in registers: slot p sits in lane p%32,
 //     register p/32.  The few candidates of a batch are compacted in shared
 //     memory and inserted or placed by rank, which gives the reference's
-//     result whenever no distances are equal; ties, NaN and larger counts
-//     run its comparator network (bitonic batch sort, pool/batch merge,
+//     result whenever they are distinct; ties, NaN and larger counts run
+//     its comparator network (bitonic batch sort, pool/batch merge,
 //     half-cleaner, graph_search.cuh:888-957 and :1424-1493) on those
 //     registers, across lanes through shuffles and inside a lane for
 //     distances >= 32;
@@ -297,19 +297,22 @@ __device__ __forceinline__ void merge_pool(float (&pd)[pool_regs(NL)], int (&pi)
 // Every other batch slot holds a distance >= the pool's largest, so its
 // comparison takes nothing.  Placing each candidate against pool slot L-1-r
 // by its rank and running the half-cleaner (place_half_clean) therefore gives
-// exactly the network's pool.  If besides no candidate equals a pool slot and
-// no two pool slots (of real points) are equal, the half-cleaner's result is
-// the one ascending order of the L smallest, and the slots can be moved there
-// directly (place_direct).  Anything else -- ties, NaN, more candidates than
-// kept -- runs the reference's network, where the handling of equal keys
-// decides which id lands where.
+// exactly the network's pool, ties with or within the pool included.  Anything
+// else -- equal candidates, NaN, more candidates than kept -- runs the
+// reference's network, where the handling of equal keys decides which id lands
+// where.
 //
 // The candidates are compacted in shared memory and ranked one or two per
 // lane against broadcast reads: about 2 instructions per candidate, where
 // ranking them in the batch's slots by shuffles took 15 to 90, and no wide
 // network in the usual case.  On one GB300 this took the 256-slot pools
 // (10k queries, 500k x 96, BF16, beam 256, width 4) with the filter below from
-// 3.80 to 2.5 ms.
+// 3.80 to 2.5 ms.  Moving the pool's slots straight to their merged places, by
+// comparing each candidate with the one register it falls into, was slower in
+// every pool it was made for, as its loop over the candidates is serial: 128
+// slots FP32 300 queries 416 / 321 us with the half-cleaner, 10k 2.63 / 2.24
+// ms; BF16 2,049 queries 576 / 512 us; 256 slots FP32 300 queries 498 / 357 us,
+// BF16 10k 2.77 / 2.64 ms.
 template <int NL, int NB>
 __host__ __device__ constexpr int cands_per_lane() { return batch_regs(NB) >= 4 ? 2 : 1; }
 template <int NL, int NB>
@@ -321,6 +324,8 @@ __host__ __device__ constexpr int cand_limit() {
 // Candidates that are inserted one by one instead of ranked (pools of one or
 // two registers).
 constexpr int kInsertMax = 4;
+template <int NL>
+__host__ __device__ constexpr bool inserts() { return pool_regs(NL) <= 2; }
 
 // One candidate into the sorted pool; eq is set if a slot equals it.
 template <int NL>
@@ -384,7 +389,7 @@ __device__ __forceinline__ int rank_candidates(float (&pd)[pool_regs(NL)], int (
   }
   if (m == 0) return 0;
   if (__any_sync(kFull, nan)) return -1;
-  if constexpr (PR <= 2) {
+  if constexpr (inserts<NL>()) {
     // One to four candidates are inserted one after the other: every slot
     // above the candidate moves up by one.  Without ties this is again the
     // one ascending order of the L smallest; with one, the pool is put back.
@@ -526,12 +531,6 @@ __device__ __forceinline__ void place_half_clean(float (&pd)[pool_regs(NL)], int
   half_clean<NL>(pd, pi, lane);
 }
 
-// Pools of 4 registers and more are merged directly: their half-cleaner is
-// 5 shuffle stages over every register, against two moves through shared
-// memory here.
-template <int NL>
-__host__ __device__ constexpr bool direct_pool() { return pool_regs(NL) >= 4; }
-
 // True when two neighbouring slots of the sorted pool hold equal distances
 // of real points.
 template <int NL>
@@ -550,83 +549,6 @@ __device__ __forceinline__ bool pool_has_ties(const float (&pd)[pool_regs(NL)], 
     tie |= prev == pd[j] && pd[j] != kMaxDist;
   }
   return __any_sync(kFull, tie);
-}
-
-// Moves the pool's slots and the m ranked candidates to their places in the
-// merged ascending order (the first L are kept).  Each candidate falls into
-// one pool register, found against the registers' last slots, and is compared
-// with that register alone; registers below the first candidate's stay as
-// they are.  Returns false, changing nothing, if a candidate equals a pool
-// slot.
-template <int NL, int NB>
-__device__ __forceinline__ bool place_direct(float (&pd)[pool_regs(NL)], int (&pi)[pool_regs(NL)], int* s_ids,
-                                             float* s_dist, int m, int lane) {
-  constexpr int L = pool_slots(NL), PR = pool_regs(NL), KC = cands_per_lane<NL, NB>();
-  float cv[KC];
-  int ci[KC], cp[KC], reg[KC];
-#pragma unroll
-  for (int t = 0; t < KC; ++t) {
-    const int r = 32 * t + lane;
-    cv[t] = r < m ? s_dist[r] : __int_as_float(0x7f800000);
-    ci[t] = r < m ? s_ids[r] : 0;
-    cp[t] = L;
-    reg[t] = r < m ? 0 : PR;
-  }
-#pragma unroll
-  for (int j = 0; j < PR - 1; ++j) {
-    const float last = __shfl_sync(kFull, pd[j], 31);
-#pragma unroll
-    for (int t = 0; t < KC; ++t) reg[t] += last < cv[t] ? 1 : 0;
-  }
-  int cnt[PR];        // candidates below each pool slot
-  int upto[PR];       // candidates in registers 0..j
-  bool eq = false;
-#pragma unroll
-  for (int j = 0; j < PR; ++j) {
-    int hi = 0;
-#pragma unroll
-    for (int t = 0; t < KC; ++t) hi += __popc(__ballot_sync(kFull, reg[t] <= j));
-    upto[j] = hi;
-    const int lo = j > 0 ? upto[j > 0 ? j - 1 : 0] : 0;
-    cnt[j] = lo;
-#pragma unroll 1
-    for (int r = lo; r < hi; ++r) {
-      const float c = s_dist[r];
-      const bool below = c < pd[j];
-      cnt[j] += below ? 1 : 0;
-      eq |= c == pd[j];
-      const int place = 32 * j + r + __popc(__ballot_sync(kFull, !below));
-#pragma unroll
-      for (int t = 0; t < KC; ++t)
-        if (32 * t + lane == r) cp[t] = place;
-    }
-  }
-  if (__any_sync(kFull, eq)) return false;
-  __syncwarp();  // every lane has read the candidates
-#pragma unroll
-  for (int t = 0; t < KC; ++t)
-    if (cp[t] < L) {
-      s_dist[cp[t]] = cv[t];
-      s_ids[cp[t]] = ci[t];
-    }
-#pragma unroll
-  for (int j = 0; j < PR; ++j) {
-    if (upto[j] == 0) continue;
-    const int p = 32 * j + lane + cnt[j];
-    if (p < L) {
-      s_dist[p] = pd[j];
-      s_ids[p] = pi[j];
-    }
-  }
-  __syncwarp();
-#pragma unroll
-  for (int j = 0; j < PR; ++j) {
-    if (upto[j] == 0) continue;
-    pd[j] = s_dist[32 * j + lane];
-    pi[j] = s_ids[32 * j + lane];
-  }
-  __syncwarp();
-  return true;
 }
 
 // Partial sum of one lane for one row: s = t0*t0, then fmaf(tc, tc, s) over
@@ -1298,15 +1220,12 @@ __device__ __forceinline__ void merge_batch(float (&pd)[pool_regs(NL)], int (&pi
                                             int* s_ids, float* s_dist, int m, unsigned slots, bool& ties,
                                             int lane) {
   if (m == 0) return;
-  if constexpr (direct_pool<NL>()) {
-    if (m > 0 && !ties && place_direct<NL, NB>(pd, pi, s_ids, s_dist, m, lane)) return;
-  }
   if (m > 0)
     place_half_clean<NL, NB>(pd, pi, s_ids, s_dist, m, lane);
   else
     merge_network<NL, NB>(pd, pi, np, s_ids, s_dist, slots, lane);
   __syncwarp();
-  ties = pool_has_ties<NL>(pd, lane);
+  if constexpr (inserts<NL>()) ties = pool_has_ties<NL>(pd, lane);
 }
 
 // Exact FP32 rerank of the final pool for the reduced-precision paths: the
