@@ -7,8 +7,9 @@
 //     (B = 32*NB slots) live in registers: slot p sits in lane p%32,
 //     register p/32.  The few candidates of a batch are compacted in shared
 //     memory and inserted or placed by rank, which gives the reference's
-//     result whenever they are distinct; ties, NaN and larger counts run
-//     its comparator network (bitonic batch sort, pool/batch merge,
+//     result whenever they are distinct and the pool is sorted; ties, larger
+//     counts, and all batches of a query from its first NaN on run its
+//     comparator network (bitonic batch sort, pool/batch merge,
 //     half-cleaner, graph_search.cuh:888-957 and :1424-1493) on those
 //     registers, across lanes through shuffles and inside a lane for
 //     distances >= 32;
@@ -302,6 +303,14 @@ __device__ __forceinline__ void merge_pool(float (&pd)[pool_regs(NL)], int (&pi)
 // reference's network, where the handling of equal keys decides which id lands
 // where.
 //
+// All of this needs a pool that is sorted ascending.  A batch with a NaN breaks
+// that: no comparison with it swaps, so the batch sort, and then the pool, may
+// come out in any order (a NaN itself never enters the pool, as pool > NaN is
+// false).  From a query's first such batch that reaches the network on, all of
+// its batches go through the network (kPoolUnsorted).  Checking the pool and
+// going back once it is sorted again would serve only such queries, and cost
+// the others: 10k queries at beam 256 and width 4 2.48 ms instead of 2.39.
+//
 // The candidates are compacted in shared memory and ranked one or two per
 // lane against broadcast reads: about 2 instructions per candidate, where
 // ranking them in the batch's slots by shuffles took 15 to 90, and no wide
@@ -355,14 +364,20 @@ __device__ __forceinline__ void insert_one(float (&pd)[pool_regs(NL)], int (&pi)
   }
 }
 
-// Merges the batch's candidates, (s_dist, s_ids)[0, n) below pmax, as far as
-// that can be done here: none or a few inserted ones leave the pool done and
-// give 0; otherwise they are compacted, ranked and left sorted ascending in
-// slots [0, m), padded with +inf to a multiple of four, and m is returned; or
-// -1, pool and arrays as they were, if the network has to run.
+// A search's loop state, in one register (a register of its own for the flag
+// made kernels spill): the iterations since the visited filter's last rebuild,
+// and whether the pool may be out of order.
+constexpr int kRebuildAge = 7;    // mask of the count
+constexpr int kPoolUnsorted = 8;  // a slot may be above the next one
+
+// Merges the batch's candidates, (s_dist, s_ids)[0, n) below pmax, into a
+// sorted pool, as far as that can be done here: none or a few inserted ones
+// leave the pool done and give 0; otherwise they are compacted, ranked and left
+// sorted ascending in slots [0, m), padded with +inf to a multiple of four, and
+// m is returned; or -1, pool and arrays as they were, if the network has to run.
 template <int NL, int NB>
 __device__ __forceinline__ int rank_candidates(float (&pd)[pool_regs(NL)], int (&pi)[pool_regs(NL)], int* s_ids,
-                                               float* s_dist, int n, float pmax, bool ties, int lane) {
+                                               float* s_dist, int n, float pmax, bool ties, int& state, int lane) {
   constexpr int PR = pool_regs(NL);
   constexpr int KC = cands_per_lane<NL, NB>();
   constexpr int kLim = cand_limit<NL, NB>();
@@ -388,7 +403,10 @@ __device__ __forceinline__ int rank_candidates(float (&pd)[pool_regs(NL)], int (
     m += __popc(__ballot_sync(kFull, d < pmax));
   }
   if (m == 0) return 0;
-  if (__any_sync(kFull, nan)) return -1;
+  if (__any_sync(kFull, nan)) {
+    state |= kPoolUnsorted;
+    return -1;
+  }
   if constexpr (inserts<NL>()) {
     // One to four candidates are inserted one after the other: every slot
     // above the candidate moves up by one.  Without ties this is again the
@@ -1348,7 +1366,7 @@ __device__ __forceinline__ void search_query(const SearchArgs& a, int q, int lan
   uint32_t tmp_flag = L >= 32 ? 0xFFFFFFFFu : ((1u << L) - 1u);  // (1 << min(L,32)) - 1 (:969)
   int iteration = 0;
   bool cz = false;  // this lane's check_zero (:967)
-  int hash_iteration = 0;
+  int state = 0;  // kRebuildAge and kPoolUnsorted
   int iter = 0;
 
   auto scan = [&](int chunk) -> uint32_t {  // :1019-1028, :1495-1510
@@ -1651,7 +1669,9 @@ __device__ __forceinline__ void search_query(const SearchArgs& a, int q, int lan
     // the pool's largest distance: lane 31 of the last register, or lane 15
     // of the 16-slot pool
     const float pmax = __shfl_sync(kFull, pd[PR - 1], NL == 0 ? 15 : 31);
-    const int m = rank_candidates<NL, NB>(pd, pi, s_ids, s_dist, n, pmax, ties, lane);
+    const int m = __builtin_expect((state & kPoolUnsorted) != 0, 0)
+                      ? -1
+                      : rank_candidates<NL, NB>(pd, pi, s_ids, s_dist, n, pmax, ties, state, lane);
     merge_batch<NL, NB>(pd, pi, np, s_ids, s_dist, m, slots, ties, lane);
     if (entry) continue;
 
@@ -1664,7 +1684,7 @@ __device__ __forceinline__ void search_query(const SearchArgs& a, int q, int lan
         break;
       }
     }
-    if (hash_iteration == 4) {  // rebuild from the pool (:1518-1529)
+    if ((state & kRebuildAge) == 4) {  // rebuild from the pool (:1518-1529)
       __syncwarp();
       bloom.clear(lane);
       __syncwarp();
@@ -1675,9 +1695,9 @@ __device__ __forceinline__ void search_query(const SearchArgs& a, int q, int lan
         bloom.add((uint32_t)id, id < np ? 1u : 0u);
       }
       __syncwarp();
-      hash_iteration = 0;
+      state &= ~kRebuildAge;
     }
-    hash_iteration++;
+    ++state;
     if (!any) break;
   }
 
