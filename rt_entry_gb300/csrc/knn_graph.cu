@@ -283,16 +283,29 @@ __global__ void __launch_bounds__(256) rerank_rows(const float* __restrict__ x, 
     for (int k = threadIdx.x + 1; k < R; k += blockDim.x) out[gi * R + k] = si[k];
 }
 
-// Row i of dst = row `rows[i]` (or i * stride) of src, in 16-byte pieces: one
-// warp per row.
+// The i-th of S sampled rows of n: one row of [i n / S, (i + 1) n / S), at a
+// place within it that multiplicative hashing (Knuth) of i gives.  A fixed
+// stride would miss whole groups of a base whose rows come in turns (24
+// clusters in turn, stride 24: every row's threshold but one cluster's came
+// from a foreign cluster, its list overflowed, and 100k x 64 took 160 ms
+// instead of 10).
+__device__ __forceinline__ int64_t sampled_row(int64_t i, int64_t S, int64_t n) {
+  const int64_t lo = i * n / S, width = (i + 1) * n / S - lo;
+  unsigned long long h = (unsigned long long)(i + 1) * 0x9e3779b97f4a7c15ull;
+  h = (h ^ (h >> 32)) * 0x9e3779b97f4a7c15ull;
+  return lo + (int64_t)(((h >> 32) * (unsigned long long)width) >> 32);
+}
+
+// Row i of dst = row rows[i] (or the i-th sampled row of `total`) of src, in
+// 16-byte pieces: one warp per row.
 __global__ void gather_split_rows(const uint4* __restrict__ src, int64_t pieces, const int64_t* __restrict__ rows,
-                                  int64_t stride, int64_t n, uint4* __restrict__ dst,
+                                  int64_t total, int64_t n, uint4* __restrict__ dst,
                                   const float* __restrict__ nrm, float* __restrict__ dnrm) {
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t i = warp; i < n; i += nwarps) {
-    const int64_t r = rows ? rows[i] : i * stride;
+    const int64_t r = rows ? rows[i] : sampled_row(i, n, total);
     for (int64_t c = lane; c < pieces; c += 32) dst[i * pieces + c] = __ldg(src + r * pieces + c);
     if (dnrm && lane == 0) dnrm[i] = nrm[r];
   }
@@ -638,7 +651,6 @@ extern "C" rte_status rte_knn_graph(const float* base, int64_t n, int d, int deg
     // distance at degree 32, and the kept count spreads by a third.
     const int64_t want = 4 * (int64_t)degree + 96;
     const int64_t S = std::min<int64_t>(std::max<int64_t>(n / 24, 256), 65536);
-    const int64_t stride = n / S;
     const int rank = (int)std::max<int64_t>(8, (want * S + n - 1) / n) + 1;  // the row itself may be sampled
     const int cap = degree <= 64 ? 1024 : 2048;
     int kmax = 64;
@@ -653,7 +665,7 @@ extern "C" rte_status rte_knn_graph(const float* base, int64_t n, int d, int deg
     RTE_CUDA(cnt.alloc((size_t)mb * 4, st));
     RTE_CUDA(list.alloc((size_t)mb * cap * sizeof(KnnHit), st));
     gather_split_rows<<<(unsigned)std::min<int64_t>((S + 7) / 8, 4096), 256, 0, st>>>(
-        B.as<uint4>(), 3 * (int64_t)dp * 2 / 16, nullptr, stride, S, Bs.as<uint4>(), n32.as<float>(),
+        B.as<uint4>(), 3 * (int64_t)dp * 2 / 16, nullptr, n, S, Bs.as<uint4>(), n32.as<float>(),
         ns.as<float>());
     RTE_CUDA(cudaGetLastError());
     const size_t fin_smem = (size_t)kFinRows * (12 * (size_t)kmax + 4 * (size_t)cap);
