@@ -406,6 +406,13 @@ rte_status rte_locate_multi(rte_index* idx, const float* projected, int64_t nq, 
  * graph from a file (graph.cu:120); no counterpart. */
 rte_status rte_knn_graph(const float* base, int64_t n, int d, int degree, int device, int32_t* graph,
                          void* stream);
+/* How rte_knn_graph works on a base of n rows (host only, for checking the
+ * rule over sizes): plan[0] whether the thresholded tensor-core pass serves
+ * it (otherwise every row's dot products are stored), [1] the columns sampled
+ * for the rows' thresholds, [2] the rank in that sample that is a threshold,
+ * [3] the columns a row's list holds, [4] the rows per launch, [5] the shared
+ * memory of a block that finishes rows, in bytes. */
+rte_status rte_knn_graph_plan(int64_t n, int degree, int64_t plan[6]);
 
 /* Limit of the bounded waits in the tensor-core kernels (the learned head,
  * its GEMMs and the tensor-core projection), in mbarrier try_wait rounds:

@@ -32,7 +32,7 @@ EXPORTS = (
     "rte_get_kdtree", "rte_index_save", "rte_index_load_dir", "rte_index_free", "rte_last_error",
     "rte_kdtree_build_host", "rte_sym_eig_host", "rte_get_search_base_lowp", "rte_gemm_bf16",
     "rte_default_train_params", "rte_learned_train", "rte_learned_predict", "rte_mlp_grad_check",
-    "rte_search_projected_noalloc", "rte_gemm_bf16_bias_argmax", "rte_mlp_head_argmax", "rte_knn_graph", "rte_locate_multi", "rte_batcher_create", "rte_batcher_search", "rte_batcher_k",
+    "rte_search_projected_noalloc", "rte_gemm_bf16_bias_argmax", "rte_mlp_head_argmax", "rte_knn_graph", "rte_knn_graph_plan", "rte_locate_multi", "rte_batcher_create", "rte_batcher_search", "rte_batcher_k",
     "rte_batcher_free", "rte_autotune", "rte_set_wait_limit", "rte_index_load_reference",
     "rte_read_vectors", "rte_index_prepare", "rte_index_release", "rte_scratch_pool_usage",
 )
@@ -128,6 +128,7 @@ def load_library(path: str = LIB_PATH):
         "rte_gemm_bf16_bias_argmax": ([P, P, P, i32, i32, i32, P, P], i32),
         "rte_mlp_head_argmax": ([P, i32, i32, P, P, P, P, P, P, i32, i32, i32, P, P], i32),
         "rte_knn_graph": ([P, i64, i32, i32, i32, P, P], i32),
+        "rte_knn_graph_plan": ([i64, i32, P], i32),
         "rte_locate_multi": ([P, P, i64, i32, P, P], i32),
         "rte_default_train_params": ([ctypes.POINTER(TrainParams)], None),
         "rte_learned_train": ([P, P, i64, ctypes.POINTER(TrainParams), ctypes.POINTER(TrainReport)], i32),
@@ -269,6 +270,13 @@ def knn_graph(base, degree: int, device: int = 0):
     po, ko = _ptr(out)
     _check(load_library().rte_knn_graph(pb, n, d, degree, device, po, None))
     return out
+
+
+def knn_graph_plan(n: int, degree: int) -> dict:
+    """How knn_graph works on a base of n rows (host only)."""
+    out = np.zeros(6, np.int64)
+    _check(load_library().rte_knn_graph_plan(n, degree, out.ctypes.data_as(ctypes.c_void_p)))
+    return dict(zip(("thresholded", "sample", "rank", "cap", "block", "smem"), (int(v) for v in out)))
 
 
 def gemm_bf16_bias_argmax(a_bits, b_bits, bias):

@@ -57,10 +57,52 @@ constexpr int kSelT = 16;                         // candidates kept per thread
 constexpr int kSelPool = kSelThreads * kSelT;     // 4096 merged per row
 constexpr int kMaxCand = 1024;                    // the retry's candidate count
 
-// The thresholded pass serves degrees of up to 128 (lists of 2048) and bases
-// of at least 1024 rows; below, the dot products in memory take less.
+// The thresholded pass serves degrees of up to 128 and bases of at least 1024
+// rows; below, the dot products in memory take less.
 constexpr int kFilterMaxDegree = 128;
 constexpr int64_t kFilterMinRows = 1024;
+constexpr int kFinRows = 8;  // rows per block of finish_rows
+
+// Sizes of the thresholded pass.
+struct FilterPlan {
+  bool use;        // false: stored products for every row
+  int64_t sample;  // columns sampled for the thresholds
+  int rank;        // a row's threshold: its rank-th smallest sampled distance
+  int cap;         // list slots per row
+  int kmax;        // candidates per row that finish_rows measures
+  int64_t block;   // rows per launch
+};
+
+size_t finish_smem(int cap, int kmax) { return (size_t)kFinRows * (12 * (size_t)kmax + 4 * (size_t)cap); }
+
+FilterPlan filter_plan(int64_t n, int degree) {
+  FilterPlan p{};
+  if (degree > kFilterMaxDegree || n < kFilterMinRows) return p;
+  // About `want` columns are kept per row: enough that the R-th smallest plus
+  // twice the error bound lies well below the threshold.  The sample is a 24th
+  // of the base, so the threshold is about its 10th smallest distance at degree
+  // 32, and the kept count spreads by a third.  It keeps growing with the base
+  // (up to 524,288 columns, whose block of dot products takes 8.6 GB): held at
+  // 65,536, 628,083 of 5M x 32 rows' lists overflowed and their dot products
+  // were stored, 27.4 s in all, now none and 18.2 s.
+  const int64_t want = 4 * (int64_t)degree + 96;
+  p.sample = std::min<int64_t>(std::max<int64_t>(n / 24, 256), 524288);
+  p.rank = (int)std::max<int64_t>(8, (want * p.sample + n - 1) / n) + 1;  // the row itself may be sampled
+  p.kmax = 64;
+  while (p.kmax < 2 * degree + 32) p.kmax <<= 1;
+  // The count of columns below the rank-th smallest of the sample has mean
+  // rank n / sample and a relative spread of 1 / sqrt(rank): a list holds four
+  // spreads more, and the slots reserved and not used.
+  const double kept = (double)n / (double)p.sample * (p.rank + 4.0 * std::sqrt((double)p.rank) + 4.0) + 128.0;
+  p.cap = degree <= 64 ? 1024 : 2048;
+  while (p.cap < kept && p.cap < 4096) p.cap <<= 1;  // 180 KB of shared memory at degree 128
+  p.use = p.cap >= kept;  // past about 90M rows most lists would overflow
+  // rows per launch: dot products with the sample of up to 1 GB, and of 4096
+  // rows at least (the pass reads the whole base for each block)
+  p.block = std::min<int64_t>(16384, std::max<int64_t>(4096, ((1ll << 30) / (p.sample * 4)) / 128 * 128));
+  p.block = std::min<int64_t>(p.block, n);
+  return p;
+}
 
 constexpr int kMeanSlices = 256;  // row slices of the column mean's first pass
 
@@ -378,7 +420,6 @@ __global__ void __launch_bounds__(256) sample_threshold(const float* __restrict_
 // unit here (1.25 TFLOP/s), and a warp per row would leave a second, nearly
 // empty round for every row -- each summing in dimension order, and every
 // warp sorts its row.
-constexpr int kFinRows = 8;
 __global__ void __launch_bounds__(32 * kFinRows) finish_rows(
     const float* __restrict__ x, int d, int64_t r0, int64_t m, const KnnHit* __restrict__ list,
     const int* __restrict__ cnt, int cap, const float* __restrict__ tau, const double* __restrict__ nrm64,
@@ -603,6 +644,21 @@ rte_status stored_rows(const float* x, int64_t n, int d, int dp, int degree, con
 
 using namespace rte;
 
+extern "C" rte_status rte_knn_graph_plan(int64_t n, int degree, int64_t* plan) {
+  clear_error();
+  if (!plan) return fail(RTE_EINVAL, "NULL argument");
+  if (n <= 0 || n >= INT32_MAX || degree <= 0 || degree > 256 || n <= degree)
+    return fail(RTE_EINVAL, "degree must be in [1, min(256, n - 1)]");
+  const FilterPlan p = filter_plan(n, degree);
+  plan[0] = p.use;
+  plan[1] = p.sample;
+  plan[2] = p.rank;
+  plan[3] = p.cap;
+  plan[4] = p.block;
+  plan[5] = p.use ? (int64_t)finish_smem(p.cap, p.kmax) : 0;
+  return RTE_OK;
+}
+
 extern "C" rte_status rte_knn_graph(const float* base, int64_t n, int d, int degree, int device,
                                     int32_t* graph, void* stream) {
   clear_error();
@@ -644,19 +700,10 @@ extern "C" rte_status rte_knn_graph(const float* base, int64_t n, int d, int deg
       n64.as<double>(), max_nrm);
   RTE_CUDA(cudaGetLastError());
   std::vector<int64_t> left;  // rows for step 4
-  if (degree <= kFilterMaxDegree && n >= kFilterMinRows) {
-    // About `want` columns are kept per row: enough that the R-th smallest
-    // plus twice the error bound lies well below the threshold.  The sample
-    // is a 24th of the base, so the threshold is about its 10th smallest
-    // distance at degree 32, and the kept count spreads by a third.
-    const int64_t want = 4 * (int64_t)degree + 96;
-    const int64_t S = std::min<int64_t>(std::max<int64_t>(n / 24, 256), 65536);
-    const int rank = (int)std::max<int64_t>(8, (want * S + n - 1) / n) + 1;  // the row itself may be sampled
-    const int cap = degree <= 64 ? 1024 : 2048;
-    int kmax = 64;
-    while (kmax < 2 * degree + 32) kmax <<= 1;
-    int64_t mb = std::min<int64_t>(16384, std::max<int64_t>(128, ((1ll << 30) / (S * 4)) / 128 * 128));
-    mb = std::min<int64_t>(mb, n);
+  const FilterPlan fp = filter_plan(n, degree);
+  if (fp.use) {
+    const int64_t S = fp.sample, mb = fp.block;
+    const int cap = fp.cap, kmax = fp.kmax;
     AsyncBuf Bs, ns, D, tau, cnt, list;
     RTE_CUDA(Bs.alloc((size_t)S * 3 * dp * 2, st));
     RTE_CUDA(ns.alloc((size_t)S * 4, st));
@@ -668,7 +715,7 @@ extern "C" rte_status rte_knn_graph(const float* base, int64_t n, int d, int deg
         B.as<uint4>(), 3 * (int64_t)dp * 2 / 16, nullptr, n, S, Bs.as<uint4>(), n32.as<float>(),
         ns.as<float>());
     RTE_CUDA(cudaGetLastError());
-    const size_t fin_smem = (size_t)kFinRows * (12 * (size_t)kmax + 4 * (size_t)cap);
+    const size_t fin_smem = finish_smem(cap, kmax);
     RTE_CUDA(cudaFuncSetAttribute(finish_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fin_smem));
     for (int64_t r0 = 0; r0 < n; r0 += mb) {
       const int64_t m = std::min(mb, n - r0);
@@ -685,7 +732,7 @@ extern "C" rte_status rte_knn_graph(const float* base, int64_t n, int d, int deg
       ga.err = err;
       RTE_CUDA(gemm_bf16_tn(ga, st));
       sample_threshold<<<(unsigned)((m + 7) / 8), 256, 0, st>>>(D.as<float>(), S, m, n32.as<float>() + r0,
-                                                                ns.as<float>(), rank, tau.as<float>());
+                                                                ns.as<float>(), fp.rank, tau.as<float>());
       RTE_CUDA(cudaGetLastError());
       RTE_CUDA(cudaMemsetAsync(cnt.p, 0, (size_t)m * 4, st));
       KnnFilterArgs f{};
