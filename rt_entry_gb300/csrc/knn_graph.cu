@@ -73,6 +73,8 @@ struct FilterPlan {
   int64_t block;   // rows per launch
 };
 
+constexpr int kMaxCap = 4096;     // list slots per row at most
+constexpr int kMaxFinish = 512;   // candidates per row that finish_rows measures at most
 size_t finish_smem(int cap, int kmax) { return (size_t)kFinRows * (12 * (size_t)kmax + 4 * (size_t)cap); }
 
 FilterPlan filter_plan(int64_t n, int degree) {
@@ -89,13 +91,13 @@ FilterPlan filter_plan(int64_t n, int degree) {
   p.sample = std::min<int64_t>(std::max<int64_t>(n / 24, 256), 524288);
   p.rank = (int)std::max<int64_t>(8, (want * p.sample + n - 1) / n) + 1;  // the row itself may be sampled
   p.kmax = 64;
-  while (p.kmax < 2 * degree + 32) p.kmax <<= 1;
+  while (p.kmax < 2 * degree + 32) p.kmax <<= 1;  // kMaxFinish at degree 128
   // The count of columns below the rank-th smallest of the sample has mean
   // rank n / sample and a relative spread of 1 / sqrt(rank): a list holds four
   // spreads more, and the slots reserved and not used.
   const double kept = (double)n / (double)p.sample * (p.rank + 4.0 * std::sqrt((double)p.rank) + 4.0) + 128.0;
   p.cap = degree <= 64 ? 1024 : 2048;
-  while (p.cap < kept && p.cap < 4096) p.cap <<= 1;  // 180 KB of shared memory at degree 128
+  while (p.cap < kept && p.cap < kMaxCap) p.cap <<= 1;  // 180 KB of shared memory at degree 128
   p.use = p.cap >= kept;  // past about 90M rows most lists would overflow
   // rows per launch: dot products with the sample of up to 1 GB, and of 4096
   // rows at least (the pass reads the whole base for each block)
@@ -716,7 +718,10 @@ extern "C" rte_status rte_knn_graph(const float* base, int64_t n, int d, int deg
         ns.as<float>());
     RTE_CUDA(cudaGetLastError());
     const size_t fin_smem = finish_smem(cap, kmax);
-    RTE_CUDA(cudaFuncSetAttribute(finish_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fin_smem));
+    // the same limit in every call: it belongs to the kernel, and a build of a
+    // smaller degree on another thread must not lower it under this one
+    RTE_CUDA(cudaFuncSetAttribute(finish_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)finish_smem(kMaxCap, kMaxFinish)));
     for (int64_t r0 = 0; r0 < n; r0 += mb) {
       const int64_t m = std::min(mb, n - r0);
       const uint16_t* Ar = A.as<uint16_t>() + r0 * 3 * dp;
