@@ -227,21 +227,34 @@ __global__ void __launch_bounds__(kSelThreads) select_rows(const float* __restri
     ki[s] = INT32_MAX;
   }
   const float* row = D + (int64_t)r * ld;
-  for (int64_t j = threadIdx.x; j < n; j += kSelThreads) {
-    const float a = __fmaf_rn(-2.0f, __ldg(row + j), __fadd_rn(qn, __ldg(nrm32 + j)));
-    if (a < kd[kSelT - 1]) {  // insert, keeping the list sorted (ties keep scan order)
-      float cd = a;
-      int ci = (int)j;
+  // Eight columns' loads are in flight ahead of the insertions, in code: left to
+  // the compiler the loop took 76 ms in one form and 90 ms in another that only
+  // loads qn differently (100k x 64, degree 129: the whole build 134 and 147 ms,
+  // 132 ms now; four columns ahead 161 ms).
+  constexpr int kAhead = 8;
+  for (int64_t j0 = threadIdx.x; j0 < n; j0 += kSelThreads * kAhead) {
+    float a[kAhead];
 #pragma unroll
-      for (int s = 0; s < kSelT; ++s)
-        if (cd < kd[s]) {
-          const float t = kd[s];
-          kd[s] = cd;
-          cd = t;
-          const int u = ki[s];
-          ki[s] = ci;
-          ci = u;
-        }
+    for (int u = 0; u < kAhead; ++u) {
+      const int64_t j = j0 + kSelThreads * u;
+      a[u] = j < n ? __fmaf_rn(-2.0f, __ldg(row + j), __fadd_rn(qn, __ldg(nrm32 + j))) : INFINITY;
+    }
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      if (a[u] < kd[kSelT - 1]) {  // insert, keeping the list sorted (ties keep scan order)
+        float cd = a[u];
+        int ci = (int)(j0 + kSelThreads * u);
+#pragma unroll
+        for (int s = 0; s < kSelT; ++s)
+          if (cd < kd[s]) {
+            const float t = kd[s];
+            kd[s] = cd;
+            cd = t;
+            const int v = ki[s];
+            ki[s] = ci;
+            ci = v;
+          }
+      }
     }
   }
   // what this thread dropped is no smaller than its last kept value (when full)
@@ -555,8 +568,11 @@ __global__ void __launch_bounds__(32 * kFinRows) finish_rows(
   for (int k = lane; k < R; k += 32) out[gi * R + k] = rid[k];
 }
 
-// Step 4 on the rows in `rows` (host): their dot products with the whole base
-// in memory, K candidates, then 1024 for those that need them.
+// Step 4 on the rows in `rows` (host, ascending): their dot products with the
+// whole base in memory, K candidates, then 1024 for those that need them.  A
+// block of dot products of more than the stream-ordered pool keeps mapped (it
+// takes up to 8 GB) is allocated apart: 200k x 64, degree 129, 350 ms from the
+// pool, which maps it anew in every call, and 342 ms.
 rte_status stored_rows(const float* x, int64_t n, int d, int dp, int degree, const uint16_t* A, const uint16_t* B,
                        const float* n32, const double* n64, const unsigned long long* max_nrm,
                        const std::vector<int64_t>& rows, int32_t* g, int* err, int64_t& n_retried, cudaStream_t st) {
@@ -567,9 +583,14 @@ rte_status stored_rows(const float* x, int64_t n, int d, int dp, int degree, con
   int64_t mb = std::max<int64_t>(128, std::min<int64_t>(8192, (int64_t)(8ll << 30) / (n * 4)));
   mb = std::min<int64_t>(mb, (int64_t)rows.size());
   const int64_t pieces = 3 * (int64_t)dp * 2 / 16;
-  AsyncBuf Af, D, cand, excl, drows, drr, loc, fl, first;
+  DevBuf<float> apart;
+  AsyncBuf pooled, Af, cand, excl, drows, drr, loc, fl;
+  if ((size_t)mb * n * 4 > kScratchKeepBytes)
+    RTE_CUDA(apart.alloc((size_t)mb * n));
+  else
+    RTE_CUDA(pooled.alloc((size_t)mb * n * 4, st));
+  float* const D = apart.p ? apart.p : pooled.as<float>();
   RTE_CUDA(Af.alloc((size_t)mb * 3 * dp * 2, st));
-  RTE_CUDA(D.alloc((size_t)mb * n * 4, st));
   RTE_CUDA(cand.alloc((size_t)mb * kMaxCand * 4, st));
   RTE_CUDA(excl.alloc((size_t)mb * 4, st));
   RTE_CUDA(drows.alloc((size_t)mb * 8, st));
@@ -581,20 +602,24 @@ rte_status stored_rows(const float* x, int64_t n, int d, int dp, int degree, con
   for (size_t b0 = 0; b0 < rows.size(); b0 += (size_t)mb) {
     const int64_t m = std::min<int64_t>(mb, (int64_t)(rows.size() - b0));
     RTE_CUDA(cudaMemcpyAsync(drows.p, rows.data() + b0, m * 8, cudaMemcpyHostToDevice, st));
-    gather_split_rows<<<(unsigned)std::min<int64_t>((m + 7) / 8, 4096), 256, 0, st>>>(
-        reinterpret_cast<const uint4*>(A), pieces, drows.as<int64_t>(), 0, m, Af.as<uint4>(), nullptr, nullptr);
     GemmArgs ga{};
-    ga.A = Af.p;
+    if (rows[b0 + m - 1] - rows[b0] == m - 1) {  // rows that follow one another: in place
+      ga.A = A + rows[b0] * 3 * dp;
+    } else {
+      gather_split_rows<<<(unsigned)std::min<int64_t>((m + 7) / 8, 4096), 256, 0, st>>>(
+          reinterpret_cast<const uint4*>(A), pieces, drows.as<int64_t>(), 0, m, Af.as<uint4>(), nullptr, nullptr);
+      ga.A = Af.p;
+    }
     ga.B = B;
     ga.M = (int)m;
     ga.N = (int)n;
     ga.K = 3 * dp;
     ga.epilogue = kEpiStoreF32;
-    ga.C = D.p;
+    ga.C = D;
     ga.ldc = (int)n;
     ga.err = err;
     RTE_CUDA(gemm_bf16_tn(ga, st));
-    select_rows<<<(unsigned)m, kSelThreads, 0, st>>>(D.as<float>(), n, drows.as<int64_t>(), n, n32, K, nullptr,
+    select_rows<<<(unsigned)m, kSelThreads, 0, st>>>(D, n, drows.as<int64_t>(), n, n32, K, nullptr,
                                                        cand.as<int32_t>(), excl.as<float>());
     RTE_CUDA(cudaGetLastError());
     RTE_CUDA(cudaMemsetAsync(fl.p, 0, 4, st));
@@ -626,7 +651,7 @@ rte_status stored_rows(const float* x, int64_t n, int d, int dp, int degree, con
     n_retried += mr;
     RTE_CUDA(cudaMemcpyAsync(loc.p, rlocal.data(), mr * 4, cudaMemcpyHostToDevice, st));
     RTE_CUDA(cudaMemcpyAsync(drr.p, rrows.data(), mr * 8, cudaMemcpyHostToDevice, st));
-    select_rows<<<(unsigned)mr, kSelThreads, 0, st>>>(D.as<float>(), n, drows.as<int64_t>(), n, n32, K2,
+    select_rows<<<(unsigned)mr, kSelThreads, 0, st>>>(D, n, drows.as<int64_t>(), n, n32, K2,
                                                         loc.as<int32_t>(), cand.as<int32_t>(), excl.as<float>());
     RTE_CUDA(cudaGetLastError());
     RTE_CUDA(cudaMemsetAsync(fl.p, 0, 4, st));
