@@ -397,6 +397,12 @@ rte_status rte_mlp_head_argmax(const uint16_t* X, int M, int dp, const uint16_t*
 rte_status rte_locate_multi(rte_index* idx, const float* projected, int64_t nq, int max_hits,
                             int32_t* out_leaves, void* stream);
 
+/* The warps per query that a search of nq queries would run with (team_warps,
+ * or the automatic choice for 0) and, if resident is not NULL, the warps that
+ * the GPU holds at once, by whose number the choice goes. */
+rte_status rte_search_team(rte_index* idx, const rte_search_params* params, int64_t nq, int* team,
+                           int64_t* resident);
+
 /* The exact degree-R kNN graph of base [n x d] (FP32, host or device): row i
  * lists the R rows j != i nearest to row i by squared L2 distance in FP64,
  * in (distance, id) order, into graph [n x R] (host or device).  Candidates

@@ -31,7 +31,7 @@ EXPORTS = (
     "rte_search_counters", "rte_index_get_info", "rte_get_pca", "rte_get_search_base",
     "rte_get_kdtree", "rte_index_save", "rte_index_load_dir", "rte_index_free", "rte_last_error",
     "rte_kdtree_build_host", "rte_sym_eig_host", "rte_get_search_base_lowp", "rte_gemm_bf16",
-    "rte_default_train_params", "rte_learned_train", "rte_learned_predict", "rte_mlp_grad_check",
+    "rte_default_train_params", "rte_learned_train", "rte_learned_predict", "rte_search_team", "rte_mlp_grad_check",
     "rte_search_projected_noalloc", "rte_gemm_bf16_bias_argmax", "rte_mlp_head_argmax", "rte_knn_graph", "rte_knn_graph_plan", "rte_locate_multi", "rte_batcher_create", "rte_batcher_search", "rte_batcher_k",
     "rte_batcher_free", "rte_autotune", "rte_set_wait_limit", "rte_index_load_reference",
     "rte_read_vectors", "rte_index_prepare", "rte_index_release", "rte_scratch_pool_usage",
@@ -129,6 +129,7 @@ def load_library(path: str = LIB_PATH):
         "rte_mlp_head_argmax": ([P, i32, i32, P, P, P, P, P, P, i32, i32, i32, P, P], i32),
         "rte_knn_graph": ([P, i64, i32, i32, i32, P, P], i32),
         "rte_knn_graph_plan": ([i64, i32, P], i32),
+        "rte_search_team": ([P, SP, i64, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int64)], i32),
         "rte_locate_multi": ([P, P, i64, i32, P, P], i32),
         "rte_default_train_params": ([ctypes.POINTER(TrainParams)], None),
         "rte_learned_train": ([P, P, i64, ctypes.POINTER(TrainParams), ctypes.POINTER(TrainReport)], i32),
@@ -505,6 +506,13 @@ class Index:
         _check(load_library().rte_search_projected(self._h, pp, ph, nq, ctypes.byref(params), pi,
                                                    pd, _stream_ptr(stream)))
         return ids, dists
+
+    def search_team(self, nq: int, params: SearchParams | None = None, **kw) -> tuple[int, int]:
+        """(warps per query of a search of nq queries, warps that the GPU holds at once)."""
+        team, resident = ctypes.c_int(), ctypes.c_int64()
+        _check(load_library().rte_search_team(self._h, ctypes.byref(self._params(params, kw)), nq,
+                                              ctypes.byref(team), ctypes.byref(resident)))
+        return team.value, resident.value
 
     def counters(self, projected, hits=None, params: SearchParams | None = None, **kw):
         """Per-query [entries_valid, expanded, dist_evals, iterations]."""

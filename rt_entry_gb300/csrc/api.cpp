@@ -241,40 +241,83 @@ int next_pow2(int v) {
 struct Plan {
   int L, k, NL, NB, wpb, grid, prec, team;
   size_t smem;
+  int64_t resident;  // warps that the GPU holds at once
   bool ordered;  // more queries than resident warps: take them in entry-leaf order
 };
 
 }  // namespace
 
 namespace rte {
-// The fewest warps per query that automatic teams use, and up to how many
-// times the resident warps a batch keeps it (one warp per query above; the
-// larger teams of small batches come on top).  A team shares the gathers, so
-// two warps keep twice the rows in flight, and the last queries of a batch
-// take half the time; the leader's own work is not shared.  Measured on one
-// GB300, queries in leaf order, ms at K = 1 / 2 / 4 warps per query:
-//   rows of more than 4 chunks in registers (960 dims, 16 warps per SM, 2
-//     rows in flight a warp): FP32 beam 64, 1k queries 2.71 / 1.87 / 1.46, 4k
-//     6.78 / 4.74 / 3.80; FP8 beam 256 width 4, 4k 9.46 / 8.70 / 8.02: four;
-//   FP32 and FP8 rows, pools of up to 64 slots, 1M x 128: beam 32, 10k
-//     queries 1.21 / 1.00 / 1.10, 50k 3.67 / 3.61 / 4.38; beam 64, 50k 6.73 /
-//     6.71 / 8.25; FP8 beam 32, 10k 1.12 / 1.04 / 1.16: two, up to ten times;
-//   FP32 beam 128: 10k queries 2.75 / 2.62 / 3.40, 20k 4.52 / 4.65 / 6.20:
-//     two, up to three times;
-//   BF16 rows (tensor-core distances): beam 32, 7k queries 0.67 / 0.60 /
-//     0.68, 10k 0.82 / 0.80 / 0.92, 20k (beam 16) 0.91 / 0.92 / 1.11; beam
-//     128, 4k 0.98 / 1.04 / 1.40: two for pools of up to 64 slots, up to
-//     twice.
-// Wider pools are bound by the leader: one.  So are FP8 rows in the kernels
-// for any chunk count (d = 256 to 768, 6k queries: 1.48 / 1.61 / 1.74 to
-// 2.22 / 2.36 / 2.50).
-TeamFloor team_floor(int prec, int C, int kernel_chunks, int L, int wpb) {
-  if (kernel_chunks > 4 && wpb % 4 == 0) return {4, 1 << 20};
-  if (wpb % 2 != 0 || L > 128) return {1, 1};
-  if (prec == kPrecBF16 && C <= 4) return L <= 64 ? TeamFloor{2, 2} : TeamFloor{1, 1};
-  if (kernel_chunks == 0 && prec == kPrecFP8) return {1, 1};
-  if (L <= 64) return {2, 10};
-  return prec == kPrecF32 && kernel_chunks != 0 ? TeamFloor{2, 3} : TeamFloor{1, 1};
+// A team shares the gathers, so two warps keep twice the rows in flight, and
+// the last queries of a batch take half the time; the leader's own work is not
+// shared.  Measured on one GB300, ms at K = 1 / 2 / 4 warps per query, queries
+// in leaf order:
+//
+// Rows of more than 4 chunks in registers (960 dims; 16 warps per SM, 2 rows in
+// flight a warp), 200k rows, degree 64, batches of 0.8, 1.6, 4.1 and 8.2 times
+// the resident warps:
+//   FP32 beam 64: 4.27 / 3.03 / 2.28, 6.86 / 4.64 / 3.80, 11.6 / 8.08 / 8.43,
+//     17.6 / 14.7 / 16.2; beam 256, width 4, 4.1 and 8.2 times: 25.1 / 17.9 /
+//     17.7, 40.0 / 31.1 / 33.5;
+//   FP8 beam 64: 2.24 / 1.80 / 1.68, 3.50 / 3.08 / 3.09, 6.58 / 6.66 / 7.23,
+//     12.4 / 13.1 / 14.2; beam 128: 2.90 / 2.43 / 2.51, 4.97 / 4.31 / 4.56,
+//     10.4 / 9.72 / 10.6; beam 256, width 4: 5.49 / 4.58 / 4.29, 8.65 / 8.14 /
+//     7.55, 16.9 / 18.6 / 17.4; beam 256, width 1, 1.6 times: 4.27 / 4.44 / 4.62;
+//   BF16 as FP8: beam 64 at 4.1 times 6.82 / 6.09 / 6.59, beam 256 width 4 at
+//     8.2 times 26.5 / 36.2 / 34.1.
+// Hence four up to twice the resident warps (one past them where a wide pool
+// meets a batch of 64), then two up to ten times for FP32 and five for pools of
+// up to 128 slots otherwise.
+//
+// Degree-16 graphs: the leader filters and merges two lists at a time, and a
+// batch has few rows to share.  100k x 128, ms at K = 1 / 2 for 0.7, 1.2, 2.1 and
+// 4.1 times the resident warps: FP32 beam 32 0.151 / 0.170, 0.247 / 0.245, 0.350
+// / 0.374, 0.628 / 0.680; BF16 beam 32 0.143 / 0.169, 0.258 / 0.243, 0.354 /
+// 0.368, 0.611 / 0.665; FP8 beam 64 0.301 / 0.342, 0.461 / 0.524, 0.768 / 0.839,
+// 1.42 / 1.58; FP32 beam 128 0.430 / 0.493, 0.700 / 0.743, 1.13 / 1.21, 2.02 /
+// 2.27.  256 dims, beam 32: FP32 0.281 / 0.286, 0.486 / 0.422, 0.667 / 0.663, 1.18
+// / 1.25, BF16 0.297 / 0.295, 0.562 / 0.478, 0.750 / 0.805, 1.34 / 1.64.  Two only
+// where one makes a second round that two fill, FP32 and BF16 pools of up to 64.
+//
+// BF16 rows of up to 4 chunks (tensor-core distances), 1M x 128, degree 64:
+// beam 32, 7k queries 0.67 / 0.60 / 0.68, 10k 0.82 / 0.80 / 0.92, 20k (beam 16)
+// 0.91 / 0.92 / 1.11; beam 128, 4k 0.98 / 1.04 / 1.40: two for pools of up to
+// 64 slots, up to twice.  Below the resident warps two make a second round where
+// one makes none, which beam 16 (degree 32, 3,506 queries: 4 to 15 % slower) and
+// the 64-dim rows of the any-dimension kernels (5 to 20 %) do not win back.
+//
+// FP32 and FP8 rows, pools of up to 64 slots, 1M x 128, degree 64: beam 32, 10k
+// queries 1.21 / 1.00 / 1.10, 50k 3.67 / 3.61 / 4.38; beam 64, 50k 6.73 / 6.71 /
+// 8.25; FP8 beam 32, 10k 1.12 / 1.04 / 1.16: two, up to ten times.  FP8 rows of 4
+// chunks over lists of 32 are the exception (200k x 128, 3,506 to 20k queries: 1
+// to 8 % slower with two).  FP32 beam 128: 10k 2.75 / 2.62 / 3.40, 20k 4.52 / 4.65
+// / 6.20: two, up to three times; rows of 1 or 2 chunks are too short for it (64
+// dims, 3,506 queries: 11 % slower).
+//
+// The kernels for any chunk count, time with two relative to one, 160 to 1000
+// dims, degrees 32 and 64.  BF16, pools of up to 64 slots: 3,506 queries 0.85 to
+// 1.09, 6,000 0.82 to 0.98, 10,000 0.88 to 1.05, 20,000 1.08 to 1.21: up to twice.
+// FP32: 10,000 0.85 to 1.01, 20,000 1.08 at beam 16, 0.92 to 1.05 at beams 32 and
+// 64, 50,000 0.96 to 0.98 there: up to three and ten times.  FP8: 6k queries 1.48
+// / 1.61 / 1.74 ms at 256 dims to 2.22 / 2.36 / 2.50 at 768: one.
+//
+// Wider pools are bound by the leader: one.
+TeamFloor team_floor(int prec, int C, int kernel_chunks, int R, int L, int B, int wpb) {
+  const TeamFloor one{};
+  const auto two = [](int load, int from = 0) { return TeamFloor{2, load, 1, 0, from}; };
+  if (kernel_chunks > 4 && wpb % 4 == 0) {
+    if (prec == kPrecF32) return TeamFloor{4, 2, 2, 10};
+    return L <= 128 ? TeamFloor{4, 2, 2, 5} : TeamFloor{4, B <= 64 ? 1 : 2};
+  }
+  if (wpb % 2 != 0 || L > 128) return one;
+  if (R == 16) return prec != kPrecFP8 && L <= 64 ? two(2, 1) : one;
+  if (prec == kPrecBF16) {
+    if (L > 64) return one;
+    return C <= 4 && (L == 16 || kernel_chunks == 0) ? two(2, 1) : two(2);
+  }
+  if (prec == kPrecFP8) return kernel_chunks != 0 && L <= 64 && (C < 4 || R >= 64) ? two(10) : one;
+  if (L <= 64) return two(kernel_chunks == 0 && L == 16 ? 3 : 10);
+  return kernel_chunks > 2 ? two(3) : one;
 }
 }  // namespace rte
 
@@ -342,11 +385,10 @@ rte_status plan_search(const rte_index* x, const rte_search_params* prm, int64_t
   if (occ <= 0)
     return fail(RTE_EINVAL, "no kernel instantiation for beam " + std::to_string(pl.L) + ", batch " +
                                 std::to_string(B) + ", precision " + std::to_string(pl.prec));
-  const int64_t resident = (int64_t)x->num_sms * occ * pl.wpb;  // warps
+  const int64_t resident = pl.resident = (int64_t)x->num_sms * occ * pl.wpb;
   pl.team = team;
   if (team == 0) {  // automatic: spread a small batch's queries over the idle warps
-    const TeamFloor f = team_floor(pl.prec, x->C, kc, pl.L, pl.wpb);
-    pl.team = nq > f.load * resident ? 1 : f.warps;
+    pl.team = team_floor(pl.prec, x->C, kc, x->degree, pl.L, B, pl.wpb).at(nq, resident);
     while (pl.team < 8 && pl.wpb % (2 * pl.team) == 0 && nq * 2 * pl.team <= resident) pl.team *= 2;
   }
   const int64_t need = (nq * pl.team + pl.wpb - 1) / pl.wpb;
@@ -606,6 +648,18 @@ void rte_default_params(rte_search_params* p) {
 }
 
 const char* rte_last_error(void) { return g_err.c_str(); }
+
+rte_status rte_search_team(rte_index* x, const rte_search_params* prm, int64_t nq, int* team, int64_t* resident) {
+  g_err.clear();
+  if (!x || !prm || !team || nq < 0) return fail(RTE_EINVAL, "bad arguments");
+  DeviceGuard guard(x->device);
+  Plan pl;
+  const rte_status s = plan_search(x, prm, nq, pl);
+  if (s != RTE_OK) return s;
+  *team = pl.team;
+  if (resident) *resident = pl.resident;
+  return RTE_OK;
+}
 
 void rte_set_wait_limit(long long rounds) { rte::tc::set_wait_limit(rounds); }
 

@@ -10,6 +10,7 @@
 #include "host_build.h"
 #include "index_kernels.h"
 #include "rtentry.h"
+#include "search_types.h"
 
 namespace rte {
 
@@ -26,13 +27,10 @@ void* mapped_host_ptr(void* p);
 // that taking its queries in leaf order (launch_order_by_leaf) pays.
 rte_status search_plan(const rte_index* x, const rte_search_params* prm, int64_t nq, int* L, int* k,
                        int* NL, int* NB, int* wpb, int* grid, size_t* smem, int* team, bool* ordered);
-// The fewest warps per query that automatic teams use, for batches of up to
-// `load` times the resident warps (api.cpp).
-struct TeamFloor {
-  int warps;
-  int load;
-};
-TeamFloor team_floor(int prec, int C, int kernel_chunks, int L, int wpb);
+// The fewest warps per query that automatic teams use (api.cpp): rows of C
+// chunks served by a kernel for kernel_chunks (0: any), graph degree R, pool
+// of L slots, batches of B.
+TeamFloor team_floor(int prec, int C, int kernel_chunks, int R, int L, int B, int wpb);
 
 #define RTE_CUDA(call)                                                                     \
   do {                                                                                     \

@@ -44,6 +44,24 @@ struct SearchOut {
   float* dists;  // or null
 };
 
+// The fewest warps per query that automatic teams use (team_floor, api.cpp),
+// by the batch's size in units of the grid's resident warps: one up to `from`,
+// `warps` up to `load`, `next` up to `next_load`, one above.  The larger teams
+// of small batches come on top.
+struct TeamFloor {
+  int warps = 1;
+  int load = 0;
+  int next = 1;
+  int next_load = 0;
+  int from = 0;
+  RTE_HD int at(long long nq, long long resident) const {
+    return nq <= from * resident        ? 1
+           : nq <= load * resident      ? warps
+           : nq <= next_load * resident ? next
+                                        : 1;
+  }
+};
+
 struct SearchArgs {
   const float* base;        // lane-interleaved FP32 rows, stride 32*C floats
   const uint16_t* base_bf16;  // lane-interleaved BF16 rows (precision 1)
@@ -67,9 +85,9 @@ struct SearchArgs {
   const SearchOut* out_dev; // if set, the outputs' addresses are read here (graph replay)
   int C;                    // chunks of 32 dims per row (set by launch_search)
   int team;                 // warps per query: 0 or 1 alone, 2/4/8 a team, < 0 chosen
-                            // by the kernel from the live query count, at least -team
-                            // up to team_load times the grid's warps
-  int team_load;
+                            // by the kernel from the live query count, at least what
+                            // `floor` says
+  TeamFloor floor;
   int* err;                 // device word set to a non-zero code when a bounded wait runs out, or null
   const int32_t* order;     // [nq] the order in which queries are taken (a permutation), or null
   int order_min;            // the order is read only for more than this many queries

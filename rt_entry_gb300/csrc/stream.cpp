@@ -93,7 +93,8 @@ rte_status capture(rte_batcher* b) {
   // fewest per query is taken in entry-leaf order, as rte_search takes
   // one; smaller batches skip the order (the sort kernel returns at once).
   const TeamFloor floor = team_floor(b->prm.precision, x->C,
-                                     search_kernel_chunks(x->C, NL, NB, b->prm.precision, x->degree == 16), L, wpb);
+                                     search_kernel_chunks(x->C, NL, NB, b->prm.precision, x->degree == 16), x->degree,
+                                     L, b->prm.search_width * x->degree, wpb);
   const int per_query = b->prm.team_warps == 0 ? floor.warps : std::max(team, 1);
   const int64_t order_min = (int64_t)grid * wpb / per_query;
   const int32_t* order = b->dorder.p;
@@ -204,8 +205,8 @@ rte_status capture(rte_batcher* b) {
     a.max_hits = 1;
     // automatic teams follow the live batch size, which the graph reads on
     // the device; the grid, planned for the capacity, leaves them room
-    a.team = b->prm.team_warps == 0 ? -floor.warps : team;
-    a.team_load = floor.load;
+    a.team = b->prm.team_warps == 0 ? -1 : team;
+    a.floor = floor;
     // bounded waits report into the head's error word (learned entries) or
     // the word after the work counter
     a.err = learned ? reinterpret_cast<int*>(b->dzero.p + b->cap * 2) : reinterpret_cast<int*>(b->dwork.p + 1);
