@@ -403,6 +403,12 @@ rte_status rte_locate_multi(rte_index* idx, const float* projected, int64_t nq, 
 rte_status rte_search_team(rte_index* idx, const rte_search_params* params, int64_t nq, int* team,
                            int64_t* resident);
 
+/* 1 if rte_batcher_search's kernels would write an output of `bytes` bytes at
+ * `out` in place: 4-byte aligned memory of `device` within one allocation, or
+ * host memory that is page-locked throughout.  0 if they would write a buffer
+ * of the batcher's, which is then copied. */
+int rte_output_is_direct(void* out, size_t bytes, int device);
+
 /* The exact degree-R kNN graph of base [n x d] (FP32, host or device): row i
  * lists the R rows j != i nearest to row i by squared L2 distance in FP64,
  * in (distance, id) order, into graph [n x R] (host or device).  Candidates

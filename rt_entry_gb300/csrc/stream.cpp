@@ -70,16 +70,43 @@ struct rte_batcher {
 
 namespace {
 
-// The address at which kernels on `device` may write p (4-byte aligned memory
-// of that device, or page-locked host memory), or null: the caller copies.
-void* direct_output(void* p, int device) {
-  cudaPointerAttributes a;
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+// The driver's cuMemGetAddressRange, or null.
+using AddressRangeFn = int (*)(unsigned long long* base, size_t* size, unsigned long long ptr);
+AddressRangeFn address_range() {
+  static const AddressRangeFn fn = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &p, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+    }
+    return reinterpret_cast<AddressRangeFn>(p);
+  }();
+  return fn;
+}
+
+// The address at which kernels on `device` may write the `bytes` bytes from p
+// (4-byte aligned memory of that device, or page-locked host memory), or null:
+// the caller copies.  All of the bytes have to be such memory: a store past an
+// allocation, or past the page-locked part of a host buffer, would fault,
+// where a copy comes back with an error.
+void* direct_output(void* p, size_t bytes, int device) {
+  cudaPointerAttributes a, z;
+  if (bytes == 0 || cudaPointerGetAttributes(&a, p) != cudaSuccess ||
+      cudaPointerGetAttributes(&z, static_cast<char*>(p) + bytes - 1) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
-  const bool ok = (a.type == cudaMemoryTypeDevice && a.device == device) || a.type == cudaMemoryTypeHost;
-  return ok && ((uintptr_t)a.devicePointer & 3) == 0 ? a.devicePointer : nullptr;
+  if (!a.devicePointer || ((uintptr_t)a.devicePointer & 3) != 0 || z.type != a.type ||
+      z.devicePointer != static_cast<char*>(a.devicePointer) + bytes - 1)
+    return nullptr;
+  if (a.type == cudaMemoryTypeHost) return a.devicePointer;
+  if (a.type != cudaMemoryTypeDevice || a.device != device || z.device != device) return nullptr;
+  unsigned long long base = 0, at = (unsigned long long)(uintptr_t)a.devicePointer;
+  size_t size = 0;
+  const AddressRangeFn range = address_range();
+  return range && range(&base, &size, at) == 0 && at + bytes <= base + size ? a.devicePointer : nullptr;
 }
 
 rte_status capture(rte_batcher* b) {
@@ -223,6 +250,10 @@ rte_status capture(rte_batcher* b) {
 
 }  // namespace
 
+extern "C" int rte_output_is_direct(void* out, size_t bytes, int device) {
+  return out && direct_output(out, bytes, device) != nullptr;
+}
+
 extern "C" rte_status rte_batcher_create(rte_index* x, int64_t max_nq,
                                          const rte_search_params* params, rte_batcher** out) {
   clear_error();
@@ -292,8 +323,8 @@ extern "C" rte_status rte_batcher_search(rte_batcher* b, const float* queries, i
   // each query's results travel as it finishes -- instead of to a buffer that
   // two copies then move: on one GB300 twelve batches of 1 to 5,000 queries
   // took 2145 us with the copies, 2030 us without.
-  int32_t* ids = static_cast<int32_t*>(direct_output(out_ids, b->idx->device));
-  float* dists = out_dists ? static_cast<float*>(direct_output(out_dists, b->idx->device)) : nullptr;
+  int32_t* ids = static_cast<int32_t*>(direct_output(out_ids, ob, b->idx->device));
+  float* dists = out_dists ? static_cast<float*>(direct_output(out_dists, ob, b->idx->device)) : nullptr;
   // the pinned slot is free: every call ends by waiting for its stream
   b->hslot->nq = (int)nq;
   b->hslot->out.ids = ids ? ids : b->dids.p;
