@@ -1,5 +1,6 @@
 """Which outputs the batcher's kernels write in place: only memory that they
 can address to its last byte.  The decision alone; nothing is written."""
+import ctypes
 import mmap
 
 import numpy as np
@@ -34,13 +35,16 @@ def test_host_outputs_must_be_page_locked_throughout(lib, cuda):
 
 
 def test_device_outputs_must_lie_in_one_allocation(lib, cuda):
-    import torch
-    size = 32 << 20  # one segment of the allocator, of exactly this size
-    a = torch.cuda.caching_allocator_alloc(size)
+    cuda.zeros(1, device="cuda")  # the primary context is current
+    drv = ctypes.CDLL("libcuda.so.1")
+    size = 32 << 20
+    ptr = ctypes.c_uint64()
+    assert drv.cuMemAlloc_v2(ctypes.byref(ptr), ctypes.c_size_t(size)) == 0
+    a = ptr.value
     try:
         assert _direct(lib, a, size) and _direct(lib, a + size - 4, 4)
         assert not _direct(lib, a, size + 4)
         assert not _direct(lib, a + size - 4, 8)
         assert not bool(lib.rte_output_is_direct(a, size, 1))  # another device's kernels
     finally:
-        torch.cuda.caching_allocator_delete(a)
+        assert drv.cuMemFree_v2(ctypes.c_uint64(a)) == 0
