@@ -361,6 +361,23 @@ rte_status rte_mlp_grad_check(const float* X, const int32_t* labels, int M, int 
                               float* gb1, float* gW2, float* gb2, float* gW3, float* gb3,
                               float* loss);
 
+/* `steps` consecutive training steps (forward, backward, Adam at rate lr) on
+ * batches X [steps][M x d] with labels [steps][M], from the weights W = {W1,
+ * b1, W2, b2, W3, b3}; d, hidden and classes are multiples of 8.  side_streams:
+ * the independent parts of a step on side streams, as training runs them, or
+ * all on one.  grads [steps][P] and the final weights [P] hold W1, b1, W2, b2,
+ * W3, b3 one after the other; loss [steps][M].  For checking that both ways
+ * give the same bits. */
+rte_status rte_mlp_steps_check(const float* X, const int32_t* labels, int steps, int M, int d, int hidden,
+                               int classes, const float* const W[6], float lr, int side_streams,
+                               float* grads, float* weights, float* loss);
+/* Training's labels for the best points ids [n]: the class (class_of_leaf
+ * [n_leaves]) of the leaf that lists each in pids [n_leaves][cap] (entries of
+ * np and above are padding); class_of_leaf[0] for an id outside [0, np) or in
+ * no leaf.  Host arrays; for checking the kernels that make them. */
+rte_status rte_point_labels_check(const int32_t* ids, int64_t n, const int32_t* pids, int64_t n_leaves,
+                                  int cap, int64_t np, const int32_t* class_of_leaf, int32_t* labels);
+
 /* BF16 tensor-core GEMM of the learned-entry MLP (tcgen05 + TMA + TMEM):
  * C [M x N] FP32 = A [M x K] * B [N x K]^T, A and B BF16 bit patterns,
  * row-major, K a multiple of 8.  Host or device pointers.  RTE_ETIMEOUT if

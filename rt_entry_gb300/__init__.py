@@ -32,6 +32,7 @@ EXPORTS = (
     "rte_get_kdtree", "rte_index_save", "rte_index_load_dir", "rte_index_free", "rte_last_error",
     "rte_kdtree_build_host", "rte_sym_eig_host", "rte_get_search_base_lowp", "rte_gemm_bf16",
     "rte_default_train_params", "rte_learned_train", "rte_learned_predict", "rte_search_team", "rte_mlp_grad_check",
+    "rte_mlp_steps_check", "rte_point_labels_check",
     "rte_search_projected_noalloc", "rte_gemm_bf16_bias_argmax", "rte_mlp_head_argmax", "rte_knn_graph", "rte_knn_graph_plan", "rte_locate_multi", "rte_batcher_create", "rte_batcher_search", "rte_batcher_k", "rte_output_is_direct",
     "rte_batcher_free", "rte_autotune", "rte_set_wait_limit", "rte_index_load_reference",
     "rte_read_vectors", "rte_index_prepare", "rte_index_release", "rte_scratch_pool_usage",
@@ -131,6 +132,8 @@ def load_library(path: str = LIB_PATH):
         "rte_knn_graph_plan": ([i64, i32, P], i32),
         "rte_search_team": ([P, SP, i64, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int64)], i32),
         "rte_output_is_direct": ([P, ctypes.c_size_t, i32], i32),
+        "rte_mlp_steps_check": ([P, P, i32, i32, i32, i32, i32, PP, ctypes.c_float, i32, P, P, P], i32),
+        "rte_point_labels_check": ([P, i64, P, i64, i32, i64, P, P], i32),
         "rte_locate_multi": ([P, P, i64, i32, P, P], i32),
         "rte_default_train_params": ([ctypes.POINTER(TrainParams)], None),
         "rte_learned_train": ([P, P, i64, ctypes.POINTER(TrainParams), ctypes.POINTER(TrainReport)], i32),

@@ -355,6 +355,45 @@ rte_status fwd_bwd(const Mlp& m, const uint16_t* Xb, const int32_t* yb, int M, S
   return RTE_OK;
 }
 
+// The optimiser's buffers: gradients and Adam moments of every tensor.
+struct AdamState {
+  DevBuf<float> gw[3], gb[3], mw[3], vw[3], mb[3], vb[3];
+  int64_t wn[3], bn[3];
+  // Allocated, not cleared.
+  rte_status alloc(int H, int C, int dp) {
+    const int64_t w[3] = {(int64_t)H * dp, (int64_t)H * H, (int64_t)C * H}, b[3] = {H, H, C};
+    for (int l = 0; l < 3; ++l) {
+      wn[l] = w[l];
+      bn[l] = b[l];
+      for (DevBuf<float>* t : {&mw[l], &vw[l], &gw[l]}) RTE_CUDA(t->alloc(w[l]));
+      for (DevBuf<float>* t : {&mb[l], &vb[l], &gb[l]}) RTE_CUDA(t->alloc(b[l]));
+    }
+    return RTE_OK;
+  }
+  rte_status clear(int l, cudaStream_t st) {
+    for (DevBuf<float>* t : {&mw[l], &vw[l], &gw[l], &mb[l], &vb[l], &gb[l]})
+      RTE_CUDA(cudaMemsetAsync(t->p, 0, t->bytes(), st));
+    return RTE_OK;
+  }
+  // Step t (from 0) at rate lr.
+  rte_status step(const Mlp& m, int64_t t, float lr, cudaStream_t st) {
+    const float b1 = 0.9f, b2 = 0.999f;
+    AdamArgs ad{};
+    for (int l = 0; l < 3; ++l) {
+      ad.t[2 * l] = AdamTensor{m.W[l].p, gw[l].p, mw[l].p, vw[l].p, m.W16[l].p, wn[l], 0};
+      ad.t[2 * l + 1] = AdamTensor{m.b[l].p, gb[l].p, mb[l].p, vb[l].p, nullptr, bn[l], 0};
+    }
+    ad.lr = lr;
+    ad.b1 = b1;
+    ad.b2 = b2;
+    ad.eps = 1e-8f;
+    ad.c1 = 1.f / (1.f - std::pow(b1, (float)(t + 1)));
+    ad.c2 = 1.f / (1.f - std::pow(b2, (float)(t + 1)));
+    RTE_CUDA(launch_adam(ad, st));
+    return RTE_OK;
+  }
+};
+
 }  // namespace
 
 extern "C" rte_status rte_mlp_head_argmax(const uint16_t* X, int M, int dp, const uint16_t* W1,
@@ -528,7 +567,7 @@ extern "C" rte_status rte_learned_train(rte_index* x, const float* train_queries
   const int64_t wn[3] = {(int64_t)H * dp, (int64_t)H * H, Cp * H};
   const int64_t bn[3] = {H, H, Cp};
   const int fan[3] = {d, H, H};
-  DevBuf<float> mw[3], vw[3], mb[3], vb[3], gw[3], gb[3];
+  AdamState adam;
   std::mt19937 rng((uint32_t)tp->seed);
   // every random number of the first epoch while the search runs
   std::vector<float> hw[3], hb[3];
@@ -554,9 +593,9 @@ extern "C" rte_status rte_learned_train(rte_index* x, const float* train_queries
     RTE_CUDA(m.W[l].alloc(wn[l]));
     RTE_CUDA(m.W16[l].alloc(wn[l]));
     RTE_CUDA(m.b[l].alloc(bn[l]));
-    for (DevBuf<float>* b : {&mw[l], &vw[l], &gw[l]}) RTE_CUDA(b->alloc(wn[l]));
-    for (DevBuf<float>* b : {&mb[l], &vb[l], &gb[l]}) RTE_CUDA(b->alloc(bn[l]));
   }
+  s = adam.alloc(H, (int)Cp, dp);
+  if (s != RTE_OK) return s;
   // 5. per-batch buffers
   StepBufs sb;
   s = sb.alloc(M, H, (int)Cp, dp);
@@ -581,14 +620,13 @@ extern "C" rte_status rte_learned_train(rte_index* x, const float* train_queries
     RTE_CUDA(cudaMemcpy(m.W[l].p, hw[l].data(), wn[l] * 4, cudaMemcpyHostToDevice));
     RTE_CUDA(cudaMemcpy(m.b[l].p, hb[l].data(), bn[l] * 4, cudaMemcpyHostToDevice));
     RTE_CUDA(launch_f32_to_bf16(m.W[l].p, wn[l], m.W16[l].p, st));
-    for (DevBuf<float>* b : {&mw[l], &vw[l], &gw[l], &mb[l], &vb[l], &gb[l]})
-      RTE_CUDA(cudaMemsetAsync(b->p, 0, b->bytes(), st));
+    s = adam.clear(l, st);
+    if (s != RTE_OK) return s;
   }
-  float* const gwp[3] = {gw[0].p, gw[1].p, gw[2].p};
-  float* const gbp[3] = {gb[0].p, gb[1].p, gb[2].p};
+  float* const gwp[3] = {adam.gw[0].p, adam.gw[1].p, adam.gw[2].p};
+  float* const gbp[3] = {adam.gb[0].p, adam.gb[1].p, adam.gb[2].p};
   const int64_t steps_per_epoch = n / M;
   const int64_t total = steps_per_epoch * tp->epochs;
-  const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
   int64_t t = 0;
   float first_loss = -1.f, last_loss = 0.f;
   std::vector<float> hl(M);
@@ -606,20 +644,8 @@ extern "C" rte_status rte_learned_train(rte_index* x, const float* train_queries
       // Adam with a cosine decay to a tenth of the rate
       const float frac = total > 1 ? (float)t / (float)(total - 1) : 0.f;
       const float lr = tp->lr * (0.1f + 0.9f * 0.5f * (1.f + std::cos(3.14159265f * frac)));
-      const float c1 = 1.f / (1.f - std::pow(b1, (float)(t + 1)));
-      const float c2 = 1.f / (1.f - std::pow(b2, (float)(t + 1)));
-      AdamArgs ad{};
-      for (int l = 0; l < 3; ++l) {
-        ad.t[2 * l] = AdamTensor{m.W[l].p, gw[l].p, mw[l].p, vw[l].p, m.W16[l].p, wn[l], 0};
-        ad.t[2 * l + 1] = AdamTensor{m.b[l].p, gb[l].p, mb[l].p, vb[l].p, nullptr, bn[l], 0};
-      }
-      ad.lr = lr;
-      ad.b1 = b1;
-      ad.b2 = b2;
-      ad.eps = eps;
-      ad.c1 = c1;
-      ad.c2 = c2;
-      RTE_CUDA(launch_adam(ad, st));
+      s = adam.step(m, t, lr, st);
+      if (s != RTE_OK) return s;
       if (t == 0 || t == total - 1) {
         RTE_CUDA(cudaMemcpy(hl.data(), sb.loss.p, M * 4, cudaMemcpyDeviceToHost));
         double sl = 0;
@@ -784,5 +810,105 @@ extern "C" rte_status rte_mlp_grad_check(const float* X, const int32_t* labels, 
   RTE_CUDA(cudaMemcpy(gb2, gb[1].p, bn[1] * 4, cudaMemcpyDeviceToHost));
   RTE_CUDA(cudaMemcpy(gb3, gb[2].p, (size_t)classes * 4, cudaMemcpyDeviceToHost));
   if (loss) RTE_CUDA(cudaMemcpy(loss, sb.loss.p, (size_t)M * 4, cudaMemcpyDeviceToHost));
+  return RTE_OK;
+}
+
+extern "C" rte_status rte_mlp_steps_check(const float* X, const int32_t* labels, int steps, int M, int d, int hidden,
+                                          int classes, const float* const W[6], float lr, int side_streams,
+                                          float* grads, float* weights, float* loss) {
+  clear_error();
+  if (!X || !labels || !W || !grads || !weights || !loss || steps <= 0 || M <= 0 || d <= 0 || hidden <= 0 ||
+      hidden % 8 || classes <= 0 || classes % 8 || d % 8)
+    return fail(RTE_EINVAL, "bad arguments (d, hidden and classes multiples of 8)");
+  for (int i = 0; i < 6; ++i)
+    if (!W[i]) return fail(RTE_EINVAL, "NULL argument");
+  cudaStream_t st = nullptr;
+  const int H = hidden, C = classes;
+  Mlp m;
+  m.d_in = m.dp = d;
+  m.hidden = H;
+  m.classes = C;
+  AdamState adam;
+  rte_status s = adam.alloc(H, C, d);
+  if (s != RTE_OK) return s;
+  int64_t params = 0;
+  for (int l = 0; l < 3; ++l) {
+    params += adam.wn[l] + adam.bn[l];
+    RTE_CUDA(m.W[l].alloc(adam.wn[l]));
+    RTE_CUDA(m.W16[l].alloc(adam.wn[l]));
+    RTE_CUDA(m.b[l].alloc(adam.bn[l]));
+    RTE_CUDA(cudaMemcpy(m.W[l].p, W[2 * l], adam.wn[l] * 4, cudaMemcpyHostToDevice));
+    RTE_CUDA(cudaMemcpy(m.b[l].p, W[2 * l + 1], adam.bn[l] * 4, cudaMemcpyHostToDevice));
+    RTE_CUDA(launch_f32_to_bf16(m.W[l].p, adam.wn[l], m.W16[l].p, st));
+    s = adam.clear(l, st);
+    if (s != RTE_OK) return s;
+  }
+  DevBuf<float> x32, g, ls;
+  DevBuf<uint16_t> xb, Xb;
+  DevBuf<int32_t> y;
+  DevBuf<int> err;
+  StepBufs sb;
+  RTE_CUDA(x32.alloc((size_t)steps * M * d));
+  RTE_CUDA(xb.alloc((size_t)steps * M * d));
+  RTE_CUDA(Xb.alloc((size_t)M * d));
+  RTE_CUDA(y.alloc((size_t)steps * M));
+  RTE_CUDA(g.alloc((size_t)steps * params));
+  RTE_CUDA(ls.alloc((size_t)steps * M));
+  RTE_CUDA(err.alloc(1));
+  s = sb.alloc(M, H, C, d);
+  if (s != RTE_OK) return s;
+  StepStreams streams;
+  s = streams.create();
+  if (s != RTE_OK) return s;
+  RTE_CUDA(cudaMemset(err.p, 0, 4));
+  RTE_CUDA(cudaMemcpy(x32.p, X, x32.bytes(), cudaMemcpyHostToDevice));
+  RTE_CUDA(cudaMemcpy(y.p, labels, y.bytes(), cudaMemcpyHostToDevice));
+  RTE_CUDA(launch_cast_rows_bf16(x32.p, (int64_t)steps * M, d, d, 1.0f, d, xb.p, st));
+  float* const gwp[3] = {adam.gw[0].p, adam.gw[1].p, adam.gw[2].p};
+  float* const gbp[3] = {adam.gb[0].p, adam.gb[1].p, adam.gb[2].p};
+  // no host wait between the steps, and one input buffer, as in training
+  for (int t = 0; t < steps; ++t) {
+    RTE_CUDA(cudaMemcpyAsync(Xb.p, xb.p + (size_t)t * M * d, Xb.bytes(), cudaMemcpyDeviceToDevice, st));
+    s = fwd_bwd(m, Xb.p, y.p + (size_t)t * M, M, sb, gwp, gbp, err.p, st, side_streams ? &streams : nullptr);
+    if (s != RTE_OK) return s;
+    float* out = g.p + (size_t)t * params;
+    for (int l = 0; l < 3; ++l) {
+      RTE_CUDA(cudaMemcpyAsync(out, gwp[l], adam.wn[l] * 4, cudaMemcpyDeviceToDevice, st));
+      RTE_CUDA(cudaMemcpyAsync(out + adam.wn[l], gbp[l], adam.bn[l] * 4, cudaMemcpyDeviceToDevice, st));
+      out += adam.wn[l] + adam.bn[l];
+    }
+    RTE_CUDA(cudaMemcpyAsync(ls.p + (size_t)t * M, sb.loss.p, (size_t)M * 4, cudaMemcpyDeviceToDevice, st));
+    s = adam.step(m, t, lr, st);
+    if (s != RTE_OK) return s;
+  }
+  RTE_CUDA(cudaMemcpy(grads, g.p, g.bytes(), cudaMemcpyDeviceToHost));
+  RTE_CUDA(cudaMemcpy(loss, ls.p, ls.bytes(), cudaMemcpyDeviceToHost));
+  for (int l = 0; l < 3; ++l) {
+    RTE_CUDA(cudaMemcpy(weights, m.W[l].p, adam.wn[l] * 4, cudaMemcpyDeviceToHost));
+    RTE_CUDA(cudaMemcpy(weights + adam.wn[l], m.b[l].p, adam.bn[l] * 4, cudaMemcpyDeviceToHost));
+    weights += adam.wn[l] + adam.bn[l];
+  }
+  int herr = 0;
+  RTE_CUDA(cudaMemcpy(&herr, err.p, 4, cudaMemcpyDeviceToHost));
+  if (herr) return fail(RTE_ETIMEOUT, "a GEMM pipeline wait ran out");
+  return RTE_OK;
+}
+
+extern "C" rte_status rte_point_labels_check(const int32_t* ids, int64_t n, const int32_t* pids, int64_t n_leaves,
+                                             int cap, int64_t np, const int32_t* class_of_leaf, int32_t* labels) {
+  clear_error();
+  if (!ids || !pids || !class_of_leaf || !labels || n <= 0 || n_leaves <= 0 || cap <= 0 || np <= 0)
+    return fail(RTE_EINVAL, "bad arguments");
+  DevBuf<int32_t> di, dpids, dc, pc, dl;
+  RTE_CUDA(di.alloc(n));
+  RTE_CUDA(dpids.alloc((size_t)n_leaves * cap));
+  RTE_CUDA(dc.alloc(n_leaves));
+  RTE_CUDA(pc.alloc(np));
+  RTE_CUDA(dl.alloc(n));
+  RTE_CUDA(cudaMemcpy(di.p, ids, di.bytes(), cudaMemcpyHostToDevice));
+  RTE_CUDA(cudaMemcpy(dpids.p, pids, dpids.bytes(), cudaMemcpyHostToDevice));
+  RTE_CUDA(cudaMemcpy(dc.p, class_of_leaf, dc.bytes(), cudaMemcpyHostToDevice));
+  RTE_CUDA(launch_point_labels(di.p, n, dpids.p, n_leaves, cap, np, dc.p, pc.p, dl.p, nullptr));
+  RTE_CUDA(cudaMemcpy(labels, dl.p, dl.bytes(), cudaMemcpyDeviceToHost));
   return RTE_OK;
 }
