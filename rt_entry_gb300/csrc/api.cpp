@@ -248,6 +248,10 @@ struct Plan {
 }  // namespace
 
 namespace rte {
+size_t search_row_bytes(const rte_index* x, int prec) {
+  return (size_t)x->np * 32 * x->C * (prec == kPrecF32 ? 4 : prec == kPrecBF16 ? 2 : 1);
+}
+
 // A team shares the gathers, so two warps keep twice the rows in flight, and
 // the last queries of a batch take half the time; the leader's own work is not
 // shared.  Measured on one GB300, ms at K = 1 / 2 / 4 warps per query, queries
@@ -301,21 +305,40 @@ namespace rte {
 // 64, 50,000 0.96 to 0.98 there: up to three and ten times.  FP8: 6k queries 1.48
 // / 1.61 / 1.74 ms at 256 dims to 2.22 / 2.36 / 2.50 at 768: one.
 //
+// Rows read from DRAM: with one warp per query twice as many queries share L2,
+// and a group of rows waits for the one before.  BF16 rows of 3 and 4 chunks,
+// degree 32, 3k / 10k / 40k queries, one and two warps.  10M x 96: beam 64 0.55 /
+// 1.54 / 5.01 and 0.54 / 1.26 / 4.38, beam 128 width 2 1.12 / 3.23 / 10.4 and
+// 0.93 / 2.24 / 7.92, beam 256 width 4 1.63 / 4.66 / 14.9 and 1.59 / 4.35 / 15.9;
+// 3M x 96 (576 MB) beam 64 0.44 / 1.11 / 3.69 and 0.45 / 1.00 / 3.39; 10M x 128,
+// beam 256 width 4 2.23 / 6.21 / 19.7 and 1.62 / 4.21 / 15.2.  But 2M x 96 (384
+// MB), 10k: beam 64 0.66 and 0.78.  FP8 rows, beam 128 width 2, 3k / 10k / 20k: 3M
+// x 128 (384 MB) 1.08 / 2.29 / 3.91 and 0.85 / 2.22 / 4.11, 3M x 96 1.13 / 2.36 /
+// 4.00 and 0.92 / 2.17 / 4.02; but 200k x 128 0.74 / 1.82 / 3.40 and 0.75 / 1.95 /
+// 3.66.
+//
 // Wider pools are bound by the leader: one.
-TeamFloor team_floor(int prec, int C, int kernel_chunks, int R, int L, int B, int wpb) {
+constexpr size_t kFarBF16 = 512ull << 20, kFarFP8 = 256ull << 20;
+TeamFloor team_floor(int prec, int C, int kernel_chunks, int R, int L, int B, int wpb, size_t row_bytes) {
   const TeamFloor one{};
   const auto two = [](int load, int from = 0) { return TeamFloor{2, load, 1, 0, from}; };
   if (kernel_chunks > 4 && wpb % 4 == 0) {
     if (prec == kPrecF32) return TeamFloor{4, 2, 2, 10};
     return L <= 128 ? TeamFloor{4, 2, 2, 5} : TeamFloor{4, B <= 64 ? 1 : 2};
   }
-  if (wpb % 2 != 0 || L > 128) return one;
+  if (wpb % 2 != 0) return one;
+  if (prec == kPrecBF16 && kernel_chunks != 0 && R != 16 && row_bytes > kFarBF16)
+    return L <= 128 ? two(10, L == 16 ? 1 : 0) : two(kernel_chunks == 4 ? 10 : 2);
+  if (L > 128) return one;
   if (R == 16) return prec != kPrecFP8 && L <= 64 ? two(2, 1) : one;
   if (prec == kPrecBF16) {
     if (L > 64) return one;
     return C <= 4 && (L == 16 || kernel_chunks == 0) ? two(2, 1) : two(2);
   }
-  if (prec == kPrecFP8) return kernel_chunks != 0 && L <= 64 && (C < 4 || R >= 64) ? two(10) : one;
+  if (prec == kPrecFP8) {
+    if (kernel_chunks != 0 && L <= 64 && (C < 4 || R >= 64)) return two(10);
+    return kernel_chunks != 0 && row_bytes > kFarFP8 ? two(2) : one;
+  }
   if (L <= 64) return two(kernel_chunks == 0 && L == 16 ? 3 : 10);
   return kernel_chunks > 2 ? two(3) : one;
 }
@@ -388,7 +411,7 @@ rte_status plan_search(const rte_index* x, const rte_search_params* prm, int64_t
   const int64_t resident = pl.resident = (int64_t)x->num_sms * occ * pl.wpb;
   pl.team = team;
   if (team == 0) {  // automatic: spread a small batch's queries over the idle warps
-    pl.team = team_floor(pl.prec, x->C, kc, x->degree, pl.L, B, pl.wpb).at(nq, resident);
+    pl.team = team_floor(pl.prec, x->C, kc, x->degree, pl.L, B, pl.wpb, search_row_bytes(x, pl.prec)).at(nq, resident);
     while (pl.team < 8 && pl.wpb % (2 * pl.team) == 0 && nq * 2 * pl.team <= resident) pl.team *= 2;
   }
   const int64_t need = (nq * pl.team + pl.wpb - 1) / pl.wpb;

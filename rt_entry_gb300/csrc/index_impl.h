@@ -29,8 +29,10 @@ rte_status search_plan(const rte_index* x, const rte_search_params* prm, int64_t
                        int* NL, int* NB, int* wpb, int* grid, size_t* smem, int* team, bool* ordered);
 // The fewest warps per query that automatic teams use (api.cpp): rows of C
 // chunks served by a kernel for kernel_chunks (0: any), graph degree R, pool
-// of L slots, batches of B.
-TeamFloor team_floor(int prec, int C, int kernel_chunks, int R, int L, int B, int wpb);
+// of L slots, batches of B, row_bytes of rows in all.
+TeamFloor team_floor(int prec, int C, int kernel_chunks, int R, int L, int B, int wpb, size_t row_bytes);
+// Bytes of the rows that a search in `prec` reads.
+size_t search_row_bytes(const rte_index* x, int prec);
 
 #define RTE_CUDA(call)                                                                     \
   do {                                                                                     \

@@ -121,7 +121,8 @@ rte_status capture(rte_batcher* b) {
   // one; smaller batches skip the order (the sort kernel returns at once).
   const TeamFloor floor = team_floor(b->prm.precision, x->C,
                                      search_kernel_chunks(x->C, NL, NB, b->prm.precision, x->degree == 16), x->degree,
-                                     L, b->prm.search_width * x->degree, wpb);
+                                     L, b->prm.search_width * x->degree, wpb,
+                                     search_row_bytes(x, b->prm.precision));
   const int per_query = b->prm.team_warps == 0 ? floor.warps : std::max(team, 1);
   const int64_t order_min = (int64_t)grid * wpb / per_query;
   const int32_t* order = b->dorder.p;

@@ -62,6 +62,27 @@ def test_the_choice_on_both_sides_of_each_line(lib, cuda, d, R, prec, L, W, line
     assert idx.search_team(200 * res, team_warps=8, **kw)[0] == 8
 
 
+def test_rows_beyond_l2_take_two_warps(lib, cuda):
+    """2.9M x 96: 557 MB of BF16 rows and 278 MB of FP8 rows, above their lines."""
+    import torch
+
+    import rt_entry_gb300 as r
+    n = 2_900_000
+    ring = (torch.arange(n, device="cuda", dtype=torch.int32)[:, None]
+            + torch.arange(1, 33, device="cuda", dtype=torch.int32)) % n
+    idx = r.Index.from_arrays(torch.zeros((n, 96), device="cuda"), ring)
+    for prec, L, W, lines in [(1, 64, 1, [(10, 2)]), (1, 128, 2, [(10, 2)]), (1, 16, 1, [(1, 1), (10, 2)]),
+                              (1, 256, 4, [(2, 2)]), (2, 128, 1, [(2, 2)]), (2, 256, 1, []), (0, 256, 1, [])]:
+        kw = dict(beam=L, k=10, search_width=W, precision=prec, entry_mode=r.ENTRY_RANDOM)
+        _, res = idx.search_team(1, **kw)
+        below = res // 2 + 1
+        for load, warps in lines:
+            assert idx.search_team(below, **kw)[0] == warps, (prec, L)
+            assert idx.search_team(load * res, **kw)[0] == warps, (prec, L)
+            below = load * res + 1
+        assert idx.search_team(below, **kw)[0] == 1, (prec, L)
+
+
 @pytest.mark.parametrize("d,R,prec,L,loads", [
     (64, 64, 0, 16, (10,)),          # two warps, then one
     (128, 32, 1, 16, (1, 2)),        # one, two, one
