@@ -328,7 +328,7 @@ TeamFloor team_floor(int prec, int C, int kernel_chunks, int R, int L, int B, in
   }
   if (wpb % 2 != 0) return one;
   if (prec == kPrecBF16 && kernel_chunks != 0 && R != 16 && row_bytes > kFarBF16)
-    return L <= 128 ? two(10, L == 16 ? 1 : 0) : two(kernel_chunks == 4 ? 10 : 2);
+    return L <= 128 ? two(10, L == 16 ? 1 : 0) : two(kernel_chunks == 4 ? 10 : 3);
   if (L > 128) return one;
   if (R == 16) return prec != kPrecFP8 && L <= 64 ? two(2, 1) : one;
   if (prec == kPrecBF16) {

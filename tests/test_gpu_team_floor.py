@@ -72,7 +72,7 @@ def test_rows_beyond_l2_take_two_warps(lib, cuda):
             + torch.arange(1, 33, device="cuda", dtype=torch.int32)) % n
     idx = r.Index.from_arrays(torch.zeros((n, 96), device="cuda"), ring)
     for prec, L, W, lines in [(1, 64, 1, [(10, 2)]), (1, 128, 2, [(10, 2)]), (1, 16, 1, [(1, 1), (10, 2)]),
-                              (1, 256, 4, [(2, 2)]), (2, 128, 1, [(2, 2)]), (2, 256, 1, []), (0, 256, 1, [])]:
+                              (1, 256, 4, [(3, 2)]), (2, 128, 1, [(2, 2)]), (2, 256, 1, []), (0, 256, 1, [])]:
         kw = dict(beam=L, k=10, search_width=W, precision=prec, entry_mode=r.ENTRY_RANDOM)
         _, res = idx.search_team(1, **kw)
         below = res // 2 + 1
