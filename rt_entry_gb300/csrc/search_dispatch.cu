@@ -99,9 +99,14 @@ void* search_kernel_ptr(int C, int NL, int NB, int prec, bool r16, bool team) {
   return f ? f(NL, NB, r16, team) : nullptr;
 }
 
-// Rows of up to 100 MB stay in the 129 MB L2 beside the graph: their search
-// does not prefetch them.
+// Rows of up to 100 MB stay in the 129 MB L2, and their search does not prefetch
+// them, unless the graph's lists push them out.  One GB300, without and with,
+// beam 256 width 2, 1k and 10k queries: 250k x 96 FP32 (96 MB) over degree 64 (64
+// MB) 0.602 / 0.612 and 4.12 / 4.27 ms; 500k x 96 BF16 (96 MB, lists 128 MB) 0.595
+// / 0.574 and 3.55 / 3.66; 760k x 128 FP8 (97 MB, lists 195 MB) 0.902 / 0.879 and
+// 6.30 / 5.93.
 constexpr size_t kL2ResidentRows = 100ull << 20;
+constexpr size_t kL2ResidentIndex = 256ull << 20;
 
 cudaError_t launch_search(const SearchArgs& a, int C, int NL, int NB, int prec, int wpb, int grid,
                           size_t smem, cudaStream_t st) {
@@ -114,7 +119,7 @@ cudaError_t launch_search(const SearchArgs& a, int C, int NL, int NB, int prec, 
   SearchArgs args = a;
   args.C = C;
   const size_t row = 32 * (size_t)C * (prec == kPrecF32 ? 4 : prec == kPrecBF16 ? 2 : 1);
-  args.prefetch = row * (size_t)a.np > kL2ResidentRows;
+  args.prefetch = row * (size_t)a.np > kL2ResidentRows || (row + 4 * (size_t)a.R) * (size_t)a.np > kL2ResidentIndex;
   void* params[] = {&args};
   // the team kernels serve the small batches; the single-warp ones begin
   // without a dependency wait and are launched plainly
