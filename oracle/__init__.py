@@ -72,8 +72,9 @@ def build_ref_launcher(force: bool = False) -> str | None:
 
 
 def build_reference() -> bool:
-    """Compile the reference's own pieces when the reference tree exists."""
-    if not os.path.isdir(REFERENCE_TREE):
+    """Compile the reference's own pieces when the reference tree exists and
+    is not an empty mount point."""
+    if not os.path.isdir(REFERENCE_TREE) or not os.listdir(REFERENCE_TREE):
         return False
     _run(["make", "-s", "-C", os.path.join(HERE, "ref"), "-j8", f"OUT={REF_OUT}",
           f"REF={REFERENCE_TREE}"])
