@@ -281,12 +281,12 @@ size_t search_row_bytes(const rte_index* x, int prec) {
 // 1.42 / 1.58; FP32 beam 128 0.430 / 0.493, 0.700 / 0.743, 1.13 / 1.21, 2.02 /
 // 2.27.  256 dims, beam 32: FP32 0.281 / 0.286, 0.486 / 0.422, 0.667 / 0.663, 1.18
 // / 1.25, BF16 0.297 / 0.295, 0.562 / 0.478, 0.750 / 0.805, 1.34 / 1.64.  Two only
-// where one makes a second round that two fill, FP32 and BF16 pools of up to 64.
+// where one makes a second wave that two fill, FP32 and BF16 pools of up to 64.
 //
 // BF16 rows of up to 4 chunks (tensor-core distances), 1M x 128, degree 64:
 // beam 32, 7k queries 0.67 / 0.60 / 0.68, 10k 0.82 / 0.80 / 0.92, 20k (beam 16)
 // 0.91 / 0.92 / 1.11; beam 128, 4k 0.98 / 1.04 / 1.40: two for pools of up to
-// 64 slots, up to twice.  Below the resident warps two make a second round where
+// 64 slots, up to twice.  Below the resident warps two make a second wave where
 // one makes none, which beam 16 (degree 32, 3,506 queries: 4 to 15 % slower) and
 // the 64-dim rows of the any-dimension kernels (5 to 20 %) do not win back.
 //

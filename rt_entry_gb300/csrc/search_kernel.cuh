@@ -324,11 +324,14 @@ __device__ __forceinline__ void merge_pool(float (&pd)[pool_regs(NL)], int (&pi)
 // network in the usual case.  On one GB300 this took the 256-slot pools
 // (10k queries, 500k x 96, BF16, beam 256, width 4) with the filter below from
 // 3.80 to 2.5 ms.  Moving the pool's slots straight to their merged places, by
-// comparing each candidate with the one register it falls into, was slower in
-// every pool it was made for, as its loop over the candidates is serial: 128
-// slots FP32 300 queries 416 / 321 us with the half-cleaner, 10k 2.63 / 2.24
-// ms; BF16 2,049 queries 576 / 512 us; 256 slots FP32 300 queries 498 / 357 us,
-// BF16 10k 2.77 / 2.64 ms.
+// comparing each candidate with the one register it falls into, was slower on
+// bases of up to 1M rows, as its loop over the candidates is serial: 128 slots
+// FP32 300 queries 416 / 321 us with the half-cleaner, 10k 2.63 / 2.24 ms; BF16
+// 2,049 queries 576 / 512 us; 256 slots FP32 300 queries 498 / 357 us, BF16 10k
+// 2.77 / 2.64 ms.  Over 10M x 96 it was slower for FP32 and FP8 rows (5.23 / 5.07
+// and 5.78 / 5.41 ms at 256 slots, width 4), and for BF16 rows faster, 4.91 and
+// 5.90 ms, where the half-cleaner takes 4.35 ms since those rows' loads are issued
+// together (mma_group) and two warps share a query (team_floor).
 template <int NL, int NB>
 __host__ __device__ constexpr int cands_per_lane() { return batch_regs(NB) >= 4 ? 2 : 1; }
 template <int NL, int NB>
